@@ -8,6 +8,7 @@
 
 #include "kernels.h"
 #include "launch.cuh"
+#include "merkle_tensor.h"
 #include "p2_device.cuh"
 #include "poseidon2_host.h"
 
@@ -33,9 +34,22 @@ void count_launches(unsigned n) { g_launches.fetch_add(n, std::memory_order_rela
 
 cudaError_t init_poseidon2_tables() {
   cudaError_t e = upload_p2(16);
-  if (e != cudaSuccess) return e;
-  return upload_p2(24);
+  if (e == cudaSuccess) e = upload_p2(24);
+  if (e == cudaSuccess) e = init_poseidon2_tensor();
+  return e;
 }
+
+// Where the tensor-core kernels (merkle_tensor.cu) take over.  Their tiles
+// are 128 rows and 608 of them fill the GPU; a tile takes 9.2 us per width-24
+// permutation alone on its SM and 16.5 us among four, so launches of few
+// tiles per SM gain nothing over one thread per row.  Measured, tensor
+// against thread, us: 16-word rows 2^15 17.5/16.3, 2^16 23.6/28.8, 2^22
+// 909/1163; 64-word rows 2^14 42/42, 2^15 55.6/58.9, 2^22 3 550/4 912; nodes
+// 2^15 13.0/11.0, 2^16 17.8/18.8, 2^17 27.8/29.0, 2^21 330/381.
+static bool leaves_on_tensor(size_t n_rows, int row_len) {
+  return n_rows >= (row_len <= 16 ? (size_t)1 << 16 : (size_t)1 << 15);
+}
+static bool nodes_on_tensor(size_t nodes) { return nodes >= ((size_t)1 << 16); }
 
 // One row per thread; a row of ROW = 16·c words is c permutations
 // (PaddingFreeSponge: overwrite the 16 rate lanes, permute).  Base rows are
@@ -152,6 +166,11 @@ cudaError_t verify_paths(const PathDesc *d, const uint32_t *words, const uint32_
 cudaError_t hash_rows(const uint32_t *rows, size_t n_rows, int row_len, uint32_t *digests,
                       cudaStream_t st) {
   if (n_rows == 0) return cudaSuccess;
+  if (leaves_on_tensor(n_rows, row_len) && ((uintptr_t)digests & 15) == 0) {
+    hash_rows_tensor(rows, n_rows, row_len, digests, st);
+    count_launches(1);
+    return cudaGetLastError();
+  }
   const int T = 128;
   unsigned grid = (unsigned)((n_rows + T - 1) / T);
   // the fixed-width kernels use 16-byte vector loads and stores
@@ -182,6 +201,17 @@ __global__ void __launch_bounds__(128) compress_level(const uint32_t *__restrict
   uint4 *d = reinterpret_cast<uint4 *>(dst + i * 8);
   d[0] = make_uint4(s[0], s[1], s[2], s[3]);
   d[1] = make_uint4(s[4], s[5], s[6], s[7]);
+}
+
+// one level of a tree: `half` nodes from the 2 half nodes at src
+static void launch_level(const uint32_t *src, uint32_t *dst, size_t half, cudaStream_t st) {
+  if (nodes_on_tensor(half)) {
+    compress_level_tensor(src, dst, half, st);
+  } else {
+    const int T = 128;
+    launch(compress_level, (unsigned)((half + T - 1) / T), T, 0, st, src, dst, half);
+  }
+  count_launches(1);
 }
 
 // ---- width-16 permutation on a quad of lanes (latency) ----
@@ -363,16 +393,13 @@ static cudaError_t launch_subtrees(uint32_t *nodes, int log_h, int l0, int log_g
 
 cudaError_t build_tree(uint32_t *nodes, int log_h, cudaStream_t st, uint32_t *host_root,
                        unsigned int *flag, unsigned int seq) {
-  const int T = 128;
   TreeTune tune = tree_tune(log_h);
   if (!tree_tune_valid(log_h, tune)) tune = TreeTune();
   int l = 0;
   for (; l < log_h && ((size_t)1 << (log_h - l)) / 2 >= ((size_t)1 << tune.wide_log); l++) {
     size_t half = ((size_t)1 << (log_h - l)) / 2;
-    launch(compress_level, (unsigned)((half + T - 1) / T), T, 0, st,
-           nodes + level_offset_words(log_h, l), nodes + level_offset_words(log_h, l + 1),
-           half);
-    count_launches(1);
+    launch_level(nodes + level_offset_words(log_h, l), nodes + level_offset_words(log_h, l + 1),
+                 half, st);
   }
   // remaining S = log_h - l steps (S <= wide_log): G = 2^((S + split)/2)
   // subtrees, then the top
@@ -390,15 +417,12 @@ cudaError_t build_tree(uint32_t *nodes, int log_h, cudaStream_t st, uint32_t *ho
 // S - g levels, then batch CTAs climb g (each CTA holds at most 512 nodes).
 cudaError_t build_tree_batch(uint32_t *nodes, int log_h, int batch, cudaStream_t st) {
   if (batch < 1 || log_h < 0 || log_h > 30) return cudaErrorInvalidValue;
-  const int T = 128;
   const size_t B = (size_t)batch;
   int l = 0;
   for (; l < log_h && (B << (log_h - l)) / 2 >= ((size_t)1 << 15); l++) {
     size_t half = (B << (log_h - l)) / 2;
-    launch(compress_level, (unsigned)((half + T - 1) / T), T, 0, st,
-           nodes + B * level_offset_words(log_h, l),
-           nodes + B * level_offset_words(log_h, l + 1), half);
-    count_launches(1);
+    launch_level(nodes + B * level_offset_words(log_h, l),
+                 nodes + B * level_offset_words(log_h, l + 1), half, st);
   }
   const int S = log_h - l;
   if (S == 0) return cudaGetLastError();

@@ -2,6 +2,7 @@
 #include "prover.h"
 #include "debug.h"
 #include "host_math.h"
+#include "merkle_tensor.h"
 #include "svo_host.h"
 #include "verifier.h"
 
@@ -140,7 +141,15 @@ void *Context::pinned(size_t bytes) {
   }
   return pinned_;
 }
+// a kernel gave up a bounded wait: what it wrote is not valid
+static void check_kernel_waits() {
+  if (gpu::tensor_wait_failed()) throw WhirError(-2, "a hash kernel's wait ran out");
+}
 void Context::wait_stream() {
+  wait_stream_done();
+  check_kernel_waits();
+}
+void Context::wait_stream_done() {
   if (!yield_) {
     cuda_check(cudaStreamSynchronize(stream_), "stream sync");
     return;
@@ -182,6 +191,7 @@ void Context::wait_flag(unsigned int seq) {
     }
     if (yield_) std::this_thread::yield();
   }
+  check_kernel_waits();
   if (prof_on(K_SYNC)) {
     acc_ms_[K_SYNC] +=
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();

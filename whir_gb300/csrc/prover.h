@@ -148,7 +148,8 @@ class Context {
   unsigned long long d2h_bytes() const { return d2h_bytes_; }
 
  private:
-  void wait_stream();
+  void wait_stream();       // and fails if a kernel gave up a bounded wait
+  void wait_stream_done();
   int device_;
   bool yield_ = false;
   cudaEvent_t block_ev_ = nullptr;
