@@ -26,8 +26,8 @@ def _rows(oracle, log_h, row_len):
 
 
 @pytest.mark.parametrize("log_h,row_len", [
-    (14, 32), (15, 16), (15, 17), (15, 64), (16, 4), (16, 8), (16, 16), (16, 31), (16, 100),
-    (17, 16), (17, 2), (18, 48),
+    (15, 64), (16, 16), (16, 17), (16, 31), (16, 64), (16, 100), (17, 4), (17, 8), (17, 12), (17, 16),
+    (17, 2), (17, 33), (18, 48),
 ])
 def test_levels(ctx, oracle, log_h, row_len):
     rows = _rows(oracle, log_h, row_len)
@@ -37,7 +37,7 @@ def test_levels(ctx, oracle, log_h, row_len):
 
 
 def test_rows_off_the_vector_grid(ctx, oracle):
-    log_h, row_len = 16, 16
+    log_h, row_len = 17, 16
     rows = _rows(oracle, log_h, row_len)
     dev = ctx.to_device(np.concatenate([np.zeros(1, np.uint32), rows]))
     h, root = ctypes.c_void_p(), np.zeros(8, np.uint32)
@@ -48,12 +48,12 @@ def test_rows_off_the_vector_grid(ctx, oracle):
 
 
 def test_interleaved_batch(ctx, oracle):
-    # 5 x 2^14 leaves in one launch: tiles that end inside no instance
-    params, n = (17, 4, 1, 1, 1, 100), 5
-    polys = [oracle.rand_fe(40 + i, 1 << 17) for i in range(n)]
+    # 5 x 2^15 leaves in one launch
+    params, n = (18, 4, 1, 1, 1, 100), 5
+    polys = [oracle.rand_fe(40 + i, 1 << 18) for i in range(n)]
     got = W.prove_batch(ctx, params, polys, claims=0, commit_only=True)
     for i in range(n):
         w, t = W.Whir(ctx, *params), W.PoseidonWriter()
-        w.commit(t, [polys[i]], [17])
+        w.commit(t, [polys[i]], [18])
         cp = t.draw_base()
         assert got[i] == (t.finalize(), cp)

@@ -43,13 +43,17 @@ cudaError_t init_poseidon2_tables() {
 // are 128 rows and 608 of them fill the GPU; a tile takes 9.2 us per width-24
 // permutation alone on its SM and 16.5 us among four, so launches of few
 // tiles per SM gain nothing over one thread per row.  Measured, tensor
-// against thread, us: 16-word rows 2^15 17.5/16.3, 2^16 23.6/28.8, 2^22
-// 909/1163; 64-word rows 2^14 42/42, 2^15 55.6/58.9, 2^22 3 550/4 912; nodes
-// 2^15 13.0/11.0, 2^16 17.8/18.8, 2^17 27.8/29.0, 2^21 330/381.
+// against thread, us: 16-word rows 2^15 17.5/16.3, 2^16 23.6/28.8, 2^17
+// 38.6/45.4, 2^22 909/1163; 64-word rows 2^15 55.6/58.9, 2^16 74.5/107, 2^22
+// 3 550/4 912; nodes 2^16 17.8/18.8, 2^17 27.8/29.0, 2^21 330/381.  A tensor
+// launch takes an SM's whole register file and thread-per-row launches of
+// these sizes do not, so where several streams share the GPU the lines lie
+// one size above the break-even alone (32 jobs of 2^14..2^20 evaluations on
+// 8 streams: 8.95 ms, 9.1 ms with the lines one size lower).
 static bool leaves_on_tensor(size_t n_rows, int row_len) {
-  return n_rows >= (row_len <= 16 ? (size_t)1 << 16 : (size_t)1 << 15);
+  return n_rows >= (row_len <= 16 ? (size_t)1 << 17 : (size_t)1 << 16);
 }
-static bool nodes_on_tensor(size_t nodes) { return nodes >= ((size_t)1 << 16); }
+static bool nodes_on_tensor(size_t nodes) { return nodes >= ((size_t)1 << 17); }
 
 // One row per thread; a row of ROW = 16·c words is c permutations
 // (PaddingFreeSponge: overwrite the 16 rate lanes, permute).  Base rows are
