@@ -609,6 +609,139 @@ __global__ void add_pows_val_kernel(E4 *__restrict__ w, size_t n_out, int s, int
   add_pows_body<VEC>(w, n_out, s, n, tab, ScaleVal{&a});
 }
 
+// The same sum for small arrays, where one thread per output would walk its
+// points one after another and the launch would last as long as that walk
+// (72 us for 2^8 outputs and 240 points).  Lanes take the points instead: a
+// warp owns 8 consecutive outputs i0 + 8 g + j, its lane l the points l, l +
+// 32, .., and a lane steps from output to output by one product with its
+// variable, so there are no power tables.  A CTA first brings its points'
+// variables and scale_t var_t^i0 into shared memory (PL_CHUNK at a time).
+// The 32 sums of a warp (8 outputs of 4 words) end one per lane after a
+// halving exchange, 31 shuffles instead of 5 for each.  TW warps share a
+// group of 8 outputs, each with every TW-th 32 points, so that the fewest
+// outputs still spread over the GPU.
+constexpr int PL_T = 256, PL_CHUNK = 512;
+template <int TW, class VARS, class SCALE>
+__device__ __forceinline__ void pow_lanes_body(uint32_t *__restrict__ w, size_t n_out, int n,
+                                               const VARS &vars, const SCALE &scale) {
+  __shared__ E4 sS[PL_CHUNK];
+  __shared__ uint32_t sv[PL_CHUNK];
+  __shared__ uint32_t red[PL_T / 32][32];
+  constexpr int GROUPS = 8 / TW;  // groups of 8 outputs per CTA
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = warp / TW;
+  const size_t i0 = (size_t)blockIdx.x * (8 * GROUPS);
+  unsigned long long a[32];
+#pragma unroll
+  for (int q = 0; q < 32; q++) a[q] = 0;
+  for (int c0 = 0; c0 < n; c0 += PL_CHUNK) {
+    const int m = n - c0 < PL_CHUNK ? n - c0 : PL_CHUNK;
+    if (c0) __syncthreads();
+    for (int t = threadIdx.x; t < m; t += PL_T) {
+      const uint32_t v = vars(c0 + t);
+      sv[t] = v;
+      sS[t] = kb::e_scale(scale(c0 + t), kb::pow(v, i0));
+    }
+    __syncthreads();
+    int k = 0;
+    for (int t = (warp % TW) * 32 + lane; t < m; t += 32 * TW) {
+      const uint32_t v = sv[t];
+      const E4 s = sS[t];
+      uint32_t p = GROUPS > 1 ? kb::pow(v, 8 * (uint32_t)g) : kb::ONE;
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+#pragma unroll
+        for (int c = 0; c < 4; c++) a[4 * j + c] += (unsigned long long)s.c[c] * p;
+        if (j < 7) p = kb::mul(p, v);
+      }
+      if (++k == 3) {  // three products of at most p^2 on top of a folded sum
+        k = 0;
+#pragma unroll
+        for (int q = 0; q < 32; q++) a[q] = fold_2_32(a[q]);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 32; q++) a[q] = fold_2_32(a[q]);
+  }
+  uint32_t x[32];
+#pragma unroll
+  for (int q = 0; q < 32; q++) x[q] = kb::reduce_wide(a[q]);
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {  // lane l ends with the warp's sum of value l
+    const bool up = lane & o;
+#pragma unroll
+    for (int q = 0; q < o; q++) {
+      const uint32_t keep = up ? x[q + o] : x[q], send = up ? x[q] : x[q + o];
+      x[q] = kb::add(keep, __shfl_xor_sync(0xffffffffu, send, o));
+    }
+  }
+  uint32_t sum = x[0];
+  if constexpr (TW > 1) {
+    red[warp][lane] = sum;
+    __syncthreads();
+    if (warp % TW) return;
+#pragma unroll
+    for (int q = 1; q < TW; q++) sum = kb::add(sum, red[warp + q][lane]);
+  }
+  const size_t at = 4 * (i0 + 8 * g) + lane;  // word `lane` of the group's 8 outputs
+  if (at < 4 * n_out) w[at] = kb::add(w[at], sum);
+}
+struct VarPtr {
+  const uint32_t *p;
+  __device__ __forceinline__ uint32_t operator()(int t) const { return p[t]; }
+};
+struct VarVal {
+  const PowArgs *a;
+  __device__ __forceinline__ uint32_t operator()(int t) const { return a->vars[t]; }
+};
+// off: as add_pows_batch (instance blockIdx.y), or null for one instance of n points
+template <int TW>
+__global__ void __launch_bounds__(PL_T) pow_lanes_kernel(E4 *__restrict__ w, size_t n_out, int n,
+                                                         const uint32_t *__restrict__ vars,
+                                                         const E4 *__restrict__ scales,
+                                                         const int *__restrict__ off) {
+  pdl_wait();
+  int o = 0;
+  if (off) {
+    o = off[blockIdx.y];
+    n = off[blockIdx.y + 1] - o;
+  }
+  pow_lanes_body<TW>(reinterpret_cast<uint32_t *>(w + (size_t)blockIdx.y * n_out), n_out, n,
+                     VarPtr{vars + o}, ScalePtr{scales + o});
+}
+template <int TW>
+__global__ void __launch_bounds__(PL_T)
+    pow_lanes_val_kernel(E4 *__restrict__ w, size_t n_out, int n,
+                         const __grid_constant__ PowArgs a) {
+  pdl_wait();
+  pow_lanes_body<TW>(reinterpret_cast<uint32_t *>(w), n_out, n, VarVal{&a}, ScaleVal{&a});
+}
+
+// Warps per group of 8 outputs (TW), or 0 for the table kernels; total: all
+// instances' outputs.  Measured, us (tables / TW = 8, 2, 1): 2^8 outputs and
+// 240 points 72 / 3.0, 4.2, 5.9; 2^10, 240 74 / 3.1, 4.3, 6.0; 2^12, 240 71 /
+// 7.9, 4.5, 6.1; 2^13, 240 73 / 13, 6.9, 6.3; 2^15, 240 73 / 48, 22, 18; 2^16,
+// 110 16 / 77, 28, 21 (from 2^16 on a CTA of the table kernels shares its
+// high powers).  With few points the tables' walk is short and from 2^14 on
+// the exchange costs more (2^15, 1 point: 3.1 / 37, 11, 7.3; 40: 15 / 39, 13,
+// 8.9).
+static int pow_lanes_split(size_t total, int n) {
+  if (total <= ((size_t)1 << 10)) return 8;
+  if (total <= ((size_t)1 << 12)) return 2;
+  return total <= ((size_t)1 << (n >= 32 ? 15 : 13)) ? 1 : 0;
+}
+static dim3 pow_lanes_grid(size_t n_out, int tw, int batch) {
+  const size_t per = 8 * (size_t)(8 / tw);
+  return dim3((unsigned)((n_out + per - 1) / per), (unsigned)batch);
+}
+static void pow_lanes(E4 *w, size_t n_out, int tw, const uint32_t *vars, const E4 *scales, int n,
+                      const int *off, int batch, cudaStream_t st) {
+  const dim3 g = pow_lanes_grid(n_out, tw, batch);
+  if (tw == 8) launch(pow_lanes_kernel<8>, g, PL_T, 0, st, w, n_out, n, vars, scales, off);
+  else if (tw == 2) launch(pow_lanes_kernel<2>, g, PL_T, 0, st, w, n_out, n, vars, scales, off);
+  else launch(pow_lanes_kernel<1>, g, PL_T, 0, st, w, n_out, n, vars, scales, off);
+  count_launches(1);
+}
+
 // shared memory of add_pows_body: the S_t of one CTA (none without them)
 static size_t add_pows_smem(int k, int n) {
   int s = k / 2;
@@ -618,6 +751,15 @@ static size_t add_pows_smem(int k, int n) {
 cudaError_t add_pows_val(E4 *w, int k, const PowArgs &a, int n, uint32_t *tab, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   if (n > PowArgs::N || add_pows_smem(k, n) > 48 * 1024) return cudaErrorInvalidValue;
+  if (const int tw = pow_lanes_split((size_t)1 << k, n)) {
+    const size_t N = (size_t)1 << k;
+    const dim3 g = pow_lanes_grid(N, tw, 1);
+    if (tw == 8) launch(pow_lanes_val_kernel<8>, g, PL_T, 0, st, w, N, n, a);
+    else if (tw == 2) launch(pow_lanes_val_kernel<2>, g, PL_T, 0, st, w, N, n, a);
+    else launch(pow_lanes_val_kernel<1>, g, PL_T, 0, st, w, N, n, a);
+    count_launches(1);
+    return cudaGetLastError();
+  }
   int s = k / 2;
   size_t words = add_pows_scratch_words(k, n);
   launch(pow_tables_val_kernel, (unsigned)((words + 255) / 256), 256, 0, st, a, n, s, k, tab);
@@ -642,6 +784,10 @@ cudaError_t add_pows(E4 *w, int k, const uint32_t *vars, const E4 *scales, int n
   if (n == 0) return cudaSuccess;
   const size_t smem = add_pows_smem(k, n);
   if (smem > 48 * 1024) return cudaErrorInvalidValue;  // more than 3072 points
+  if (const int tw = pow_lanes_split((size_t)1 << k, n)) {
+    pow_lanes(w, (size_t)1 << k, tw, vars, scales, n, nullptr, 1, st);
+    return cudaGetLastError();
+  }
   int s = k / 2;
   size_t words = add_pows_scratch_words(k, n);
   launch(pow_tables_kernel, (unsigned)((words + 255) / 256), 256, 0, st, vars, n, s, k, tab);
@@ -676,6 +822,10 @@ cudaError_t add_pows_batch(E4 *w, int k, const uint32_t *vars, const E4 *scales,
   if (n_total == 0) return cudaSuccess;
   const size_t smem = add_pows_smem(k, max_n);
   if (smem > 48 * 1024 || batch < 1 || batch > 65535) return cudaErrorInvalidValue;
+  if (const int tw = pow_lanes_split((size_t)batch << k, max_n)) {
+    pow_lanes(w, (size_t)1 << k, tw, vars, scales, 0, off, batch, st);
+    return cudaGetLastError();
+  }
   int s = k / 2;
   size_t words = add_pows_scratch_words(k, n_total);
   launch(pow_tables_kernel, (unsigned)((words + 255) / 256), 256, 0, st, vars, n_total, s, k, tab);
