@@ -30,8 +30,8 @@ struct Publish {
 // How a tree or a DFT of a given size is split into launches.  Every choice
 // computes the same result; whir::autotune picks them by measurement.
 // Tree: levels that make >= 2^wide_log nodes run one thread per node; the
-// remaining S levels run as 2^((S + split) / 2) strided subtrees, then one
-// CTA to the root.  DFT (two-pass sizes): the first pass transforms columns
+// remaining S levels run as strided subtrees in one to three launches, the
+// first with 2^split times the default number of CTAs (merkle.cu).  DFT (two-pass sizes): the first pass transforms columns
 // of 2^L1 rows, L1 = (log_h + 1) / 2 + l1_bias.
 struct TreeTune {
   int wide_log = 15;

@@ -10,10 +10,15 @@
 #include "launch.cuh"
 #include "merkle_tensor.h"
 #include "p2_device.cuh"
+#include "p2_warp.cuh"
 #include "poseidon2_host.h"
 
 namespace whir {
 namespace gpu {
+
+// the same tables as c_p2_16 and c_p2_24, for lanes that read different entries
+__device__ uint32_t g_p2_16[8 * 16 + 20 + 16];
+__device__ uint32_t g_p2_24[8 * 24 + 23 + 24];
 
 static cudaError_t upload_p2(int width) {
   const Poseidon2Constants &c = poseidon2_constants(width);
@@ -24,8 +29,12 @@ static cudaError_t upload_p2(int width) {
     for (int i = 0; i < width; i++) buf[n++] = c.ext_rc[r][i] - kb::P;
   for (int r = 0; r < c.rounds_p; r++) buf[n++] = c.int_rc[r] - kb::P;
   for (int i = 0; i < width; i++) buf[n++] = c.diag[i];
-  if (width == 16) return cudaMemcpyToSymbol(c_p2_16, buf, n * 4);
-  return cudaMemcpyToSymbol(c_p2_24, buf, n * 4);
+  cudaError_t e = width == 16 ? cudaMemcpyToSymbol(c_p2_16, buf, n * 4)
+                              : cudaMemcpyToSymbol(c_p2_24, buf, n * 4);
+  if (e == cudaSuccess)
+    e = width == 16 ? cudaMemcpyToSymbol(g_p2_16, buf, n * 4)
+                    : cudaMemcpyToSymbol(g_p2_24, buf, n * 4);
+  return e;
 }
 
 static std::atomic<unsigned long long> g_launches{0};
@@ -53,6 +62,11 @@ cudaError_t init_poseidon2_tables() {
 static bool leaves_on_tensor(size_t n_rows, int row_len) {
   return n_rows >= (row_len <= 16 ? (size_t)1 << 17 : (size_t)1 << 16);
 }
+// And where one row per warp gives way to one per thread, which takes a
+// permutation's latency of 10.3 us per chunk however few the rows are: us,
+// warps against threads, 16-word rows 2^9 3.7/11.0, 2^11 6.1/11.1, 2^12
+// 9.0/11.2, 2^13 15.6/11.1; 64-word rows 2^9 9.9/41, 2^12 31/41, 2^13 57/41.
+static bool leaves_on_warps(size_t n_rows) { return n_rows <= ((size_t)1 << 12); }
 static bool nodes_on_tensor(size_t nodes) { return nodes >= ((size_t)1 << 17); }
 
 // One row per thread; a row of ROW = 16·c words is c permutations
@@ -84,6 +98,28 @@ __global__ void __launch_bounds__(128) hash_rows_fixed(const uint32_t *__restric
   uint4 *dst = reinterpret_cast<uint4 *>(digests + i * 8);
   dst[0] = make_uint4(s[0], s[1], s[2], s[3]);
   dst[1] = make_uint4(s[4], s[5], s[6], s[7]);
+}
+
+// One row per warp (p2_warp.cuh), any row length and alignment: a lane loads
+// its word of the next chunk before this chunk's permutation.
+__global__ void __launch_bounds__(128) hash_rows_warp(const uint32_t *__restrict__ rows,
+                                                      size_t n_rows, int row_len,
+                                                      uint32_t *__restrict__ digests) {
+  P2Warp<24> p;
+  p.init(g_p2_24);
+  pdl_wait();
+  const size_t i = (size_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+  if (i >= n_rows) return;
+  const uint32_t *row = rows + i * row_len;
+  const int l = p.lane;
+  uint32_t x = 0;
+  uint32_t next = l < 16 && l < row_len ? __ldg(row + l) : 0;
+  for (int pos = 0; pos < row_len; pos += 16) {
+    if (l < 16 && pos + l < row_len) x = next;
+    if (l < 16 && pos + 16 + l < row_len) next = __ldg(row + pos + 16 + l);
+    x = p.permute(x);
+  }
+  if (l < 8) digests[i * 8 + l] = x;
 }
 
 // Any row length (small foldings): the trailing partial chunk overwrites only
@@ -176,6 +212,11 @@ cudaError_t hash_rows(const uint32_t *rows, size_t n_rows, int row_len, uint32_t
     return cudaGetLastError();
   }
   const int T = 128;
+  if (leaves_on_warps(n_rows)) {
+    launch(hash_rows_warp, (unsigned)((n_rows + 3) / 4), T, 0, st, rows, n_rows, row_len, digests);
+    count_launches(1);
+    return cudaGetLastError();
+  }
   unsigned grid = (unsigned)((n_rows + T - 1) / T);
   // the fixed-width kernels use 16-byte vector loads and stores
   bool aligned = (((uintptr_t)rows | (uintptr_t)digests) & 15) == 0;
@@ -297,9 +338,10 @@ __device__ __forceinline__ void p2q_permute(uint32_t (&x)[4], int l, const uint3
 // log2(H/G) levels with one barrier per level, writing every level it makes
 // to the tree in global memory (the openings read them).  A narrow level is
 // bound by the latency of one permutation, so this replaces one launch per
-// level by two launches per tree (G CTAs up to the level of G nodes, then one
-// CTA, G = 1, to the root), and each node is compressed by a quad of lanes.
-// Threads: 4 per node of the first level made (at most 1024).
+// level by one to three launches per tree (G CTAs up to the level of G nodes,
+// the last with G = 1 to the root).  A level of more than warp_nodes nodes per
+// CTA is compressed by a quad of lanes per node, a smaller one by a warp per
+// node (p2_warp.cuh).
 // A batched tree (kernels.h: batch instances' leaves interleaved) is the
 // same ascent over batch 2^log_h leaves: level l holds batch 2^(log_h - l)
 // nodes at batch * level_offset_words(log_h, l), and G is a multiple of
@@ -307,8 +349,7 @@ __device__ __forceinline__ void p2q_permute(uint32_t (&x)[4], int l, const uint3
 __global__ void __launch_bounds__(1024) tree_subtrees(uint32_t *__restrict__ nodes, int log_h,
                                                      int l0, int steps, uint32_t *host_root,
                                                      unsigned int *flag, unsigned int seq,
-                                                     unsigned batch) {
-  pdl_wait();
+                                                     unsigned batch, int warp_nodes) {
   extern __shared__ uint4 sm[];  // 2 uint4 per node of this CTA's share
   __shared__ uint32_t kc[8 * 16 + 20];
   for (int i = threadIdx.x; i < 8 * 16 + 20; i += blockDim.x) kc[i] = c_p2_16[i];
@@ -316,13 +357,36 @@ __global__ void __launch_bounds__(1024) tree_subtrees(uint32_t *__restrict__ nod
   uint32_t dg[4];
 #pragma unroll
   for (int i = 0; i < 4; i++) dg[i] = c_p2_16[8 * 16 + 20 + 4 * l + i];
+  P2Warp<16> pw;
+  pw.init(g_p2_16);
+  pdl_wait();
   const size_t G = gridDim.x, j = blockIdx.x;
   int n = (int)(((size_t)batch << (log_h - l0)) / G);
   const uint4 *src = reinterpret_cast<const uint4 *>(nodes + batch * level_offset_words(log_h, l0));
   for (int q = threadIdx.x; q < 2 * n; q += blockDim.x) sm[q] = src[(j + G * (q >> 1)) * 2 + (q & 1)];
   __syncthreads();
+  uint32_t *smw = reinterpret_cast<uint32_t *>(sm);
   for (int st = 0; st < steps; st++) {
     const int half = n >> 1;
+    uint32_t *level = nodes + batch * level_offset_words(log_h, l0 + st + 1);
+    if (half <= warp_nodes) {  // one warp per node, one word per lane
+      const int wm = threadIdx.x >> 5, lane = pw.lane;
+      uint32_t y = 0;
+      if (wm < half) {
+        // lanes 0..7: the left child, 8..15: the right child
+        y = lane < 16 ? smw[lane < 8 ? 8 * wm + lane : 8 * (wm + half) + lane - 8] : 0;
+        y = pw.permute(y);
+        if (lane < 8) {
+          level[(j + G * wm) * 8 + lane] = y;
+          if (host_root && G == 1 && half == 1) host_root[lane] = y;  // the root, also to the host
+        }
+      }
+      __syncthreads();  // every read of this level's shared copy is done
+      if (wm < half && lane < 8) smw[8 * wm + lane] = y;
+      __syncthreads();
+      n = half;
+      continue;
+    }
     const bool warp_live = ((threadIdx.x & ~31) >> 2) < half;  // warp-uniform
     const bool live = m < half;
     uint32_t x[4] = {0, 0, 0, 0};
@@ -333,15 +397,8 @@ __global__ void __launch_bounds__(1024) tree_subtrees(uint32_t *__restrict__ nod
         x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
       }
       p2q_permute(x, l, kc, dg);
-      if (live && l < 2) {
-        uint4 *dst =
-            reinterpret_cast<uint4 *>(nodes + batch * level_offset_words(log_h, l0 + st + 1));
-        dst[(j + G * m) * 2 + l] = make_uint4(x[0], x[1], x[2], x[3]);
-        if (host_root && G == 1 && half == 1) {  // the root, also to the host
-#pragma unroll
-          for (int w = 0; w < 4; w++) host_root[4 * l + w] = x[w];
-        }
-      }
+      if (live && l < 2)
+        reinterpret_cast<uint4 *>(level)[(j + G * m) * 2 + l] = make_uint4(x[0], x[1], x[2], x[3]);
     }
     __syncthreads();  // every read of this level's shared copy is done
     if (live && l < 2) sm[2 * m + l] = make_uint4(x[0], x[1], x[2], x[3]);
@@ -383,16 +440,37 @@ void set_tree_tune(int log_h, TreeTune t) {
   g_tree_tune[log_h].store((t.wide_log << 4) | (t.split + 2), std::memory_order_relaxed);
 }
 
-static cudaError_t launch_subtrees(uint32_t *nodes, int log_h, int l0, int log_g, cudaStream_t st,
-                                   uint32_t *host_root, unsigned int *flag, unsigned int seq) {
-  int steps = log_h - l0 - log_g;
+// One launch of `ctas` subtrees: levels l0 .. l0 + steps of a tree (batch
+// instances).  A level of few nodes in all waits for one permutation, which
+// takes a warp 2.0 us, a quad of lanes 2.8 us; a level of many is bound by
+// instructions, of which a quad needs a quarter (per SM: 8 nodes 2.3 us on
+// warps and 2.8 on quads, 16 nodes 3.4 and 2.8).  So warps take levels of up
+// to 8 nodes per CTA and 2048 in all.
+// Threads: a quad per node made at the first step, a warp per node later.
+static cudaError_t launch_subtrees(uint32_t *nodes, int log_h, int l0, int steps, size_t ctas,
+                                   int batch, cudaStream_t st, uint32_t *host_root = nullptr,
+                                   unsigned int *flag = nullptr, unsigned int seq = 0) {
   if (steps <= 0) return cudaSuccess;
-  int n = 1 << steps;  // nodes per CTA at level l0
-  int threads = 2 * n < 32 ? 32 : 2 * n;  // a quad per node made at the first step
-  launch(tree_subtrees, 1u << log_g, threads, (size_t)n * 32, st, nodes, log_h, l0, steps,
-         host_root, flag, seq, 1u);
+  if (steps > 9 || ctas > 0x7fffffffu) return cudaErrorInvalidValue;
+  const int n = 1 << steps;  // nodes per CTA at level l0
+  int warp_nodes = 0;
+  for (int h = 1; h <= 8 && h <= n / 2 && ctas * h <= 2048; h *= 2) warp_nodes = h;
+  const int threads = std::max({2 * n, 32, 32 * warp_nodes});
+  launch(tree_subtrees, (unsigned)ctas, threads, (size_t)n * 32, st, nodes, log_h, l0, steps,
+         host_root, flag, seq, (unsigned)batch, warp_nodes);
   count_launches(1);
   return cudaGetLastError();
+}
+
+// log2 of the first launch's subtrees for a narrow part of S levels.  Up to 9
+// levels in two launches; from 10 on three, the first with up to 128 CTAs
+// (one per SM), so that all levels but the first few have at most 8 nodes per
+// CTA (a launch costs 2.5 us, a level 1.9 to 2.4 us on warps and 4.2 on
+// quads; 11 levels: 31.6 us in three launches, 34.7 in two).  A CTA starts
+// with at most 512 nodes.
+static int first_split(int S, int split) {
+  const int g = (S <= 5 ? 0 : S <= 9 ? S / 2 : std::min(7, S - 4)) + split;
+  return std::min(std::max({g, S - 9, 0}), std::min(S, 9));
 }
 
 cudaError_t build_tree(uint32_t *nodes, int log_h, cudaStream_t st, uint32_t *host_root,
@@ -405,14 +483,17 @@ cudaError_t build_tree(uint32_t *nodes, int log_h, cudaStream_t st, uint32_t *ho
     launch_level(nodes + level_offset_words(log_h, l), nodes + level_offset_words(log_h, l + 1),
                  half, st);
   }
-  // remaining S = log_h - l steps (S <= wide_log): G = 2^((S + split)/2)
-  // subtrees, then the top
-  int S = log_h - l;
-  int log_g = std::max(0, std::min(S, (S + tune.split) / 2));
-  // only the last launch (one CTA, G = 1) reaches the root
-  cudaError_t e = launch_subtrees(nodes, log_h, l, log_g, st, host_root, flag, seq);
+  // the remaining S = log_h - l steps (S <= wide_log) in up to three launches
+  const int S = log_h - l, g = first_split(S, tune.split);
+  const int g2 = g >= 6 ? g - 4 : 0;  // 16 nodes per CTA, if the top has 64 or more
+  cudaError_t e;
+  if (g == 0) return launch_subtrees(nodes, log_h, l, S, 1, 1, st, host_root, flag, seq);
+  e = launch_subtrees(nodes, log_h, l, S - g, (size_t)1 << g, 1, st);
+  if (e == cudaSuccess && g2)
+    e = launch_subtrees(nodes, log_h, log_h - g, g - g2, (size_t)1 << g2, 1, st);
   if (e != cudaSuccess) return e;
-  return launch_subtrees(nodes, log_h, log_h - log_g, 0, st, host_root, flag, seq);
+  const int top = g2 ? g2 : g;  // only the last launch (one CTA) reaches the root
+  return launch_subtrees(nodes, log_h, log_h - top, top, 1, 1, st, host_root, flag, seq);
 }
 
 // ---- batched trees (kernels.h) ----
@@ -433,18 +514,9 @@ cudaError_t build_tree_batch(uint32_t *nodes, int log_h, int batch, cudaStream_t
   int g = S / 2;
   if (S - g > 9) g = S - 9;
   if (g > 9 || (B << g) > 0x7fffffffu) return cudaErrorInvalidValue;
-  const int parts[2][2] = {{l, S - g}, {log_h - g, g}};  // (first level, steps)
-  for (int i = 0; i < 2; i++) {
-    const int l0 = parts[i][0], steps = parts[i][1];
-    if (steps == 0) continue;
-    const size_t G = B << (i == 0 ? g : 0);
-    const int n = 1 << steps;
-    const int threads = 2 * n < 32 ? 32 : 2 * n;
-    launch(tree_subtrees, (unsigned)G, threads, (size_t)n * 32, st, nodes, log_h, l0, steps,
-           nullptr, nullptr, 0, (unsigned)batch);
-    count_launches(1);
-  }
-  return cudaGetLastError();
+  const cudaError_t e = launch_subtrees(nodes, log_h, l, S - g, B << g, batch, st);
+  if (e != cudaSuccess) return e;
+  return launch_subtrees(nodes, log_h, log_h - g, g, B, batch, st);
 }
 
 __global__ void gather_openings_batch_kernel(const uint32_t *__restrict__ rows, int row_len,
