@@ -10,7 +10,7 @@
 #include "launch.cuh"
 #include "merkle_tensor.h"
 #include "p2_device.cuh"
-#include "p2_warp.cuh"
+#include "p2_lanes.cuh"
 #include "poseidon2_host.h"
 
 namespace whir {
@@ -62,11 +62,15 @@ cudaError_t init_poseidon2_tables() {
 static bool leaves_on_tensor(size_t n_rows, int row_len) {
   return n_rows >= (row_len <= 16 ? (size_t)1 << 17 : (size_t)1 << 16);
 }
-// And where one row per warp gives way to one per thread, which takes a
-// permutation's latency of 10.3 us per chunk however few the rows are: us,
-// warps against threads, 16-word rows 2^9 3.7/11.0, 2^11 6.1/11.1, 2^12
-// 9.0/11.2, 2^13 15.6/11.1; 64-word rows 2^9 9.9/41, 2^12 31/41, 2^13 57/41.
-static bool leaves_on_warps(size_t n_rows) { return n_rows <= ((size_t)1 << 12); }
+// Lanes per row of small launches (0: one thread).  A thread takes a
+// permutation's latency of 10.3 us per chunk however few the rows are, a quad
+// of lanes 4.4 us, a warp 2.1 us; the instructions grow the other way.  us,
+// warp / quad / thread: 16-word rows 2^9 3.8/6.0/11.0, 2^11 6.1/6.0/11.1, 2^12
+// 9.0/6.1/11.1, 2^13 16/7.7/11.0, 2^14 29/13/11.1; 64-word rows 2^9
+// 10/17.6/41, 2^11 19/17.7/41, 2^12 31/17.8/41, 2^13 56/24/41, 2^14 106/45/41.
+static int leaf_lanes(size_t n_rows) {
+  return n_rows <= ((size_t)1 << 10) ? 32 : n_rows <= ((size_t)1 << 13) ? 4 : 0;
+}
 static bool nodes_on_tensor(size_t nodes) { return nodes >= ((size_t)1 << 17); }
 
 // One row per thread; a row of ROW = 16·c words is c permutations
@@ -100,7 +104,7 @@ __global__ void __launch_bounds__(128) hash_rows_fixed(const uint32_t *__restric
   dst[1] = make_uint4(s[4], s[5], s[6], s[7]);
 }
 
-// One row per warp (p2_warp.cuh), any row length and alignment: a lane loads
+// One row per warp (p2_lanes.cuh), any row length and alignment: a lane loads
 // its word of the next chunk before this chunk's permutation.
 __global__ void __launch_bounds__(128) hash_rows_warp(const uint32_t *__restrict__ rows,
                                                       size_t n_rows, int row_len,
@@ -120,6 +124,37 @@ __global__ void __launch_bounds__(128) hash_rows_warp(const uint32_t *__restrict
     x = p.permute(x);
   }
   if (l < 8) digests[i * 8 + l] = x;
+}
+
+// One row per four lanes, any row length and alignment.
+__global__ void __launch_bounds__(128) hash_rows_quad(const uint32_t *__restrict__ rows,
+                                                      size_t n_rows, int row_len,
+                                                      uint32_t *__restrict__ digests) {
+  __shared__ uint32_t kc[P2Quad<24>::CONSTS];
+  for (int i = threadIdx.x; i < P2Quad<24>::CONSTS; i += blockDim.x) kc[i] = __ldg(g_p2_24 + i);
+  P2Quad<24> p;
+  p.init(g_p2_24, kc);
+  __syncthreads();
+  pdl_wait();
+  const size_t i = (size_t)blockIdx.x * (blockDim.x / 4) + (threadIdx.x >> 2);
+  const bool live = i < n_rows;  // a whole warp permutes together
+  const uint32_t *row = rows + (live ? i : 0) * row_len + p.l;
+  uint32_t x[6] = {0, 0, 0, 0, 0, 0}, next[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+    if (4 * j + p.l < row_len) next[j] = __ldg(row + 4 * j);
+  for (int pos = 0; pos < row_len; pos += 16) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      if (pos + 4 * j + p.l < row_len) x[j] = next[j];
+      if (pos + 16 + 4 * j + p.l < row_len) next[j] = __ldg(row + pos + 16 + 4 * j);
+    }
+    p.permute(x);
+  }
+  if (live) {
+    digests[i * 8 + p.l] = x[0];
+    digests[i * 8 + 4 + p.l] = x[1];
+  }
 }
 
 // Any row length (small foldings): the trailing partial chunk overwrites only
@@ -212,8 +247,11 @@ cudaError_t hash_rows(const uint32_t *rows, size_t n_rows, int row_len, uint32_t
     return cudaGetLastError();
   }
   const int T = 128;
-  if (leaves_on_warps(n_rows)) {
-    launch(hash_rows_warp, (unsigned)((n_rows + 3) / 4), T, 0, st, rows, n_rows, row_len, digests);
+  if (const int lanes = leaf_lanes(n_rows)) {
+    const size_t per = T / lanes;  // rows per CTA
+    const unsigned g = (unsigned)((n_rows + per - 1) / per);
+    if (lanes == 32) launch(hash_rows_warp, g, T, 0, st, rows, n_rows, row_len, digests);
+    else launch(hash_rows_quad, g, T, 0, st, rows, n_rows, row_len, digests);
     count_launches(1);
     return cudaGetLastError();
   }
@@ -259,77 +297,6 @@ static void launch_level(const uint32_t *src, uint32_t *dst, size_t half, cudaSt
   count_launches(1);
 }
 
-// ---- width-16 permutation on a quad of lanes (latency) ----
-// Lane l of an aligned group of 4 holds state words 4l .. 4l+3, which is one
-// group of the light MDS: mat4 stays in registers and a column sum is three
-// xor shuffles added as a tree (one shuffle latency, not two in a row).  In
-// an internal round every lane tracks word 0 (z), so the S-box on it runs
-// beside the shuffled sum of the other 15 words instead of before it.  The
-// round constants for the next round are loaded one round ahead.  This is
-// what a level with few nodes waits for: on GB300 one permutation takes
-// 3.1 us here against 4.9 us for two chained xor shuffles per sum with the
-// S-box ahead of the internal sum (and 6.3 us on one thread).
-constexpr unsigned FULL = 0xffffffffu;
-
-__device__ __forceinline__ uint32_t quad_sum(uint32_t v) {
-  uint32_t a = __shfl_xor_sync(FULL, v, 1, 4);
-  uint32_t b = __shfl_xor_sync(FULL, v, 2, 4);
-  uint32_t c = __shfl_xor_sync(FULL, v, 3, 4);
-  return kb::add(kb::add(v, a), kb::add(b, c));
-}
-
-__device__ __forceinline__ void p2q_mds(uint32_t (&x)[4]) {
-  p2_mat4(x[0], x[1], x[2], x[3]);
-#pragma unroll
-  for (int c = 0; c < 4; c++) x[c] = kb::add(x[c], quad_sum(x[c]));
-}
-
-// kc: the 8*16 external and 20 internal constants (stored minus p); dg: this
-// lane's 4 diagonal entries (Montgomery form).  Every lane of the warp calls it.
-__device__ __forceinline__ void p2q_permute(uint32_t (&x)[4], int l, const uint32_t *kc,
-                                            const uint32_t (&dg)[4]) {
-  using namespace kb;
-  static_assert(P2Shape<16>::RP == 20, "internal rounds");
-  static_assert(diag_entry16(0).sign < 0 && diag_entry16(0).num == 2 &&
-                    diag_entry16(0).log_den == 0,
-                "word 0's diagonal entry");
-  p2q_mds(x);
-  uint32_t ce[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) ce[i] = kc[4 * l + i];
-#pragma unroll 1
-  for (int r = 0; r < 8; r++) {
-    if (r == 4) {
-      uint32_t z = __shfl_sync(FULL, x[0], 0, 4);  // word 0 (lane 0's first)
-      uint32_t rc = kc[8 * 16];
-#pragma unroll 2
-      for (int q = 0; q < 20; q++) {
-        const uint32_t rcn = kc[8 * 16 + (q + 1 < 20 ? q + 1 : 19)];
-        const uint32_t y = sbox((int32_t)(z + rc));
-        // this lane's words other than word 0: < 4p < 2^33, folded below 2p
-        uint64_t w = (uint64_t)x[1] + x[2] + x[3] + (l ? x[0] : 0u);
-        uint32_t f = (uint32_t)(w & 0x7fffffffu) + (uint32_t)(w >> 31) * 0x00ffffffu;
-        const uint32_t sum = add(quad_sum(kb::umin(f, f - P)), y);
-        const uint32_t x0 = l ? x[0] : y;
-        x[0] = add(sum, mul(x0, dg[0]));
-#pragma unroll
-        for (int i = 1; i < 4; i++) x[i] = add(sum, mul(x[i], dg[i]));
-        z = sub(sum, dbl(y));  // word 0's diagonal entry is -2
-        rc = rcn;
-      }
-    }
-    uint32_t cn[4];
-    const int rn = r + 1 < 8 ? r + 1 : 7;
-#pragma unroll
-    for (int i = 0; i < 4; i++) cn[i] = kc[rn * 16 + 4 * l + i];
-#pragma unroll
-    for (int i = 0; i < 4; i++) x[i] = sbox((int32_t)(x[i] + ce[i]));
-    p2q_mds(x);
-#pragma unroll
-    for (int i = 0; i < 4; i++) ce[i] = cn[i];
-  }
-}
-
 // ---- the narrow levels of a tree ----
 // With halves pairing, node i of a level with H nodes is C(i, i + H/2) of the
 // level below, and i, i + H/2 agree modulo any G dividing H/2.  So the nodes
@@ -341,7 +308,7 @@ __device__ __forceinline__ void p2q_permute(uint32_t (&x)[4], int l, const uint3
 // level by one to three launches per tree (G CTAs up to the level of G nodes,
 // the last with G = 1 to the root).  A level of more than warp_nodes nodes per
 // CTA is compressed by a quad of lanes per node, a smaller one by a warp per
-// node (p2_warp.cuh).
+// node (p2_lanes.cuh).
 // A batched tree (kernels.h: batch instances' leaves interleaved) is the
 // same ascent over batch 2^log_h leaves: level l holds batch 2^(log_h - l)
 // nodes at batch * level_offset_words(log_h, l), and G is a multiple of
@@ -351,12 +318,11 @@ __global__ void __launch_bounds__(1024) tree_subtrees(uint32_t *__restrict__ nod
                                                      unsigned int *flag, unsigned int seq,
                                                      unsigned batch, int warp_nodes) {
   extern __shared__ uint4 sm[];  // 2 uint4 per node of this CTA's share
-  __shared__ uint32_t kc[8 * 16 + 20];
-  for (int i = threadIdx.x; i < 8 * 16 + 20; i += blockDim.x) kc[i] = c_p2_16[i];
-  const int l = threadIdx.x & 3, m = threadIdx.x >> 2;
-  uint32_t dg[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) dg[i] = c_p2_16[8 * 16 + 20 + 4 * l + i];
+  __shared__ uint32_t kc[P2Quad<16>::CONSTS];
+  for (int i = threadIdx.x; i < P2Quad<16>::CONSTS; i += blockDim.x) kc[i] = __ldg(g_p2_16 + i);
+  P2Quad<16> pq;
+  pq.init(g_p2_16, kc);
+  const int l = pq.l, m = threadIdx.x >> 2;
   P2Warp<16> pw;
   pw.init(g_p2_16);
   pdl_wait();
@@ -391,17 +357,23 @@ __global__ void __launch_bounds__(1024) tree_subtrees(uint32_t *__restrict__ nod
     const bool live = m < half;
     uint32_t x[4] = {0, 0, 0, 0};
     if (warp_live) {
-      if (live) {
-        // lanes 0, 1: the left child's two halves; lanes 2, 3: the right child's
-        uint4 v = l < 2 ? sm[2 * m + l] : sm[2 * (m + half) + (l - 2)];
-        x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+      if (live) {  // words l and l + 4 of the left child, then of the right one
+        x[0] = smw[8 * m + l];
+        x[1] = smw[8 * m + 4 + l];
+        x[2] = smw[8 * (m + half) + l];
+        x[3] = smw[8 * (m + half) + 4 + l];
       }
-      p2q_permute(x, l, kc, dg);
-      if (live && l < 2)
-        reinterpret_cast<uint4 *>(level)[(j + G * m) * 2 + l] = make_uint4(x[0], x[1], x[2], x[3]);
+      pq.permute(x);
+      if (live) {
+        level[(j + G * m) * 8 + l] = x[0];
+        level[(j + G * m) * 8 + 4 + l] = x[1];
+      }
     }
     __syncthreads();  // every read of this level's shared copy is done
-    if (live && l < 2) sm[2 * m + l] = make_uint4(x[0], x[1], x[2], x[3]);
+    if (live) {
+      smw[8 * m + l] = x[0];
+      smw[8 * m + 4 + l] = x[1];
+    }
     __syncthreads();
     n = half;
   }
