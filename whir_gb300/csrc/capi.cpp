@@ -372,11 +372,17 @@ int whir_combine_eqs(whir_ctx *ctx, uint32_t *weights, int k, const uint32_t *po
   size_t per = ((size_t)1 << sl) + ((size_t)1 << (k - sl));
   ctx->eq.reserve(sizeof(E4) * per * n);
   cudaStream_t st = ctx->ctx.stream();
-  for (int t = 0; t < n; t++) {
-    whir::gpu::Point z = point_in(points + (size_t)4 * k * t, k);
-    E4 *tab = ctx->eq.as<E4>() + per * t;
-    whir::cuda_check(whir::gpu::eq_split(z, sl, s, tab, tab + ((size_t)1 << sl), st), "eq_split");
-    s = kb::e_mul(s, a);
+  whir::gpu::EqArgs q;  // the tables of up to EqArgs::N points per launch
+  for (int t0 = 0; t0 < n; t0 += whir::gpu::EqArgs::N) {
+    const int m = std::min(n - t0, (int)whir::gpu::EqArgs::N);
+    for (int t = 0; t < m; t++) {
+      const whir::gpu::Point z = point_in(points + (size_t)4 * k * (t0 + t), k);
+      std::copy(z.z, z.z + k, q.z + t * whir::gpu::EqArgs::K);
+      q.scale[t] = s;
+      s = kb::e_mul(s, a);
+    }
+    whir::cuda_check(whir::gpu::eq_tables_val(q, m, k, sl, ctx->eq.as<E4>() + per * t0, st),
+                     "eq_tables");
   }
   whir::cuda_check(whir::gpu::add_eq(reinterpret_cast<E4 *>(weights), k, ctx->eq.as<E4>(), n, st),
                    "add_eq");

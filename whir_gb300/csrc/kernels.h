@@ -191,6 +191,11 @@ struct CodeState {
 // added to acc[0..8) (and, at round 0, the sum term to acc[8..12))
 cudaError_t code_round(const CodeState &s, int round, kb::E4 r_prev, unsigned long long *acc,
                        cudaStream_t st, const Publish &pub = Publish());
+// sumcheck_round (with coefficients) and code_round of one instance in one launch
+cudaError_t sumcheck_round_code(const kb::E4 *p_in, const kb::E4 *w_in, size_t n_in, bool fold,
+                                kb::E4 r, kb::E4 *p_out, kb::E4 *w_out, const CodeState &s,
+                                int round, kb::E4 r_prev, unsigned long long *acc,
+                                cudaStream_t st, const Publish &pub = Publish());
 cudaError_t code_finish(const CodeState &s, kb::E4 r_last, cudaStream_t st);
 // out[q] = <eq(rs), row(idx[q])> over base rows (fold_with_code evals, prover.rs:497-506)
 cudaError_t row_evals(const uint32_t *rows, int row_len, const uint32_t *idx, int n,

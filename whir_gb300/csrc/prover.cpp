@@ -768,28 +768,28 @@ struct Prover::Impl {
   void coeffs_begin(const gpu::CodeState *code = nullptr, int code_round = 0,
                     E4 code_r = E4{}) {
     unsigned long long *a = acc.as<unsigned long long>();
-    // the last reducing launch publishes the sums to pinned memory and
-    // re-zeroes them (no memset, no copy); with no queries (rate 1) there is
-    // no code pass and the round pass publishes
+    // the launch publishes the sums to pinned memory and re-zeroes them (no
+    // memset, no copy); with no queries (rate 1) there is no code pass
     if (code && code->n == 0) code = nullptr;
     gpu::Publish pub = publish(12);
-    gpu::Publish none;
-    size_t n = (size_t)1 << kc;
+    const size_t n = (size_t)1 << kc;
+    const bool fold = pending;
+    const size_t n_in = fold ? 2 * n : n;
+    E4 *po = fold ? sp[1 - ping].as<E4>() : nullptr, *wo = fold ? sw[1 - ping].as<E4>() : nullptr;
+    const E4 r = fold ? pending_r : e_zero();
     ctx->prof_begin(Context::K_SUMCHECK);
-    if (pending) {
-      cuda_check(gpu::sumcheck_round(P(), W(), 2 * n, true, pending_r, sp[1 - ping].as<E4>(),
-                                     sw[1 - ping].as<E4>(), true, a, st(), code ? none : pub),
+    if (code)
+      cuda_check(gpu::sumcheck_round_code(P(), W(), n_in, fold, r, po, wo, *code, code_round,
+                                          code_r, a, st(), pub),
                  "round");
+    else
+      cuda_check(gpu::sumcheck_round(P(), W(), n_in, fold, r, po, wo, true, a, st(), pub),
+                 "round");
+    if (fold) {
       ping = 1 - ping;
       pending = false;
-      ctx->prof_end(Context::K_SUMCHECK, 3.0 * 2 * 16 * (double)n);
-    } else {
-      cuda_check(gpu::sumcheck_round(P(), W(), n, false, e_zero(), nullptr, nullptr, true, a, st(),
-                                     code ? none : pub),
-                 "round");
-      ctx->prof_end(Context::K_SUMCHECK, 2 * 16 * (double)n);
     }
-    if (code) cuda_check(gpu::code_round(*code, code_round, code_r, a, st(), pub), "code_round");
+    ctx->prof_end(Context::K_SUMCHECK, (fold ? 3.0 * 2 : 2.0) * 16 * (double)n);
   }
   void flush() {
     if (!pending) return;

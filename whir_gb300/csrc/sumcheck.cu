@@ -69,18 +69,22 @@ __device__ __forceinline__ void publish_if_last(unsigned long long *acc, const P
   }
 }
 
-// eq table entries over z[off .. off+nv) times scale: entry b selects z_i
-// when bit i of b is set, 1 - z_i otherwise (Point::eq, point.rs:110-126).
-__global__ void eq_entries(Point z, int off, int nv, E4 scale, E4 *out) {
+// The split eq tables of one point: 2^s entries over z[0..s) at lo, 2^(k-s)
+// over z[s..k) times scale at hi.  Entry b selects z_i when bit i of b is
+// set, 1 - z_i otherwise (Point::eq, point.rs:110-126).
+__global__ void eq_split_kernel(const __grid_constant__ Point z, int s, E4 scale, E4 *lo, E4 *hi) {
   pdl_wait();
-  size_t b = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= ((size_t)1 << nv)) return;
-  E4 acc = scale;
+  const size_t x = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nlo = (size_t)1 << s;
+  if (x >= nlo + ((size_t)1 << (z.k - s))) return;
+  const bool low = x < nlo;
+  const size_t b = low ? x : x - nlo;
+  const int off = low ? 0 : s, nv = low ? s : z.k - s;
+  E4 acc = low ? kb::e_one() : scale;
   for (int i = 0; i < nv; i++) {
-    E4 zi = z.z[off + i];
+    const E4 zi = z.z[off + i];
     acc = kb::e_mul(acc, ((b >> i) & 1) ? zi : kb::e_sub(kb::e_one(), zi));
   }
-  out[b] = acc;
+  (low ? lo : hi)[b] = acc;
 }
 
 // n_tables split eq tables in one launch: table t = (lo: 2^s entries over
@@ -155,19 +159,12 @@ cudaError_t eq_tables_val(const EqArgs &a, int n, int k, int s, E4 *out, cudaStr
   return cudaGetLastError();
 }
 
-static cudaError_t eq_part(const Point &z, int off, int nv, E4 scale, E4 *out, cudaStream_t st) {
-  size_t n = (size_t)1 << nv;
-  unsigned T = 256, G = (unsigned)((n + T - 1) / T);
-  launch(eq_entries, G, T, 0, st, z, off, nv, scale, out);
-  count_launches(1);
-  return cudaGetLastError();
-}
-
 cudaError_t eq_split(const Point &z, int s, E4 scale, E4 *lo, E4 *hi, cudaStream_t st) {
   if (s < 0 || s > z.k) return cudaErrorInvalidValue;
-  cudaError_t e = eq_part(z, 0, s, kb::e_one(), lo, st);
-  if (e != cudaSuccess) return e;
-  return eq_part(z, s, z.k - s, scale, hi, st);
+  const size_t n = ((size_t)1 << s) + ((size_t)1 << (z.k - s));
+  launch(eq_split_kernel, (unsigned)((n + 127) / 128), 128, 0, st, z, s, scale, lo, hi);
+  count_launches(1);
+  return cudaGetLastError();
 }
 
 __global__ void eq_join(const E4 *lo, const E4 *hi, int s, size_t n, E4 *out) {
@@ -840,11 +837,9 @@ cudaError_t add_pows_batch(E4 *w, int k, const uint32_t *vars, const E4 *scales,
   return cudaGetLastError();
 }
 
-// block-wide sum of E4 values into 64-bit accumulators at acc; acc_base is
-// the launch's accumulator base for publishing (acc itself when unbatched)
+// block-wide sum of E4 values into 64-bit accumulators at acc
 template <int NV>
-__device__ __forceinline__ void block_acc(const E4 (&v)[NV], unsigned long long *acc,
-                                          unsigned long long *acc_base, const Publish &pub) {
+__device__ __forceinline__ void block_sum(const E4 (&v)[NV], unsigned long long *acc) {
   __shared__ unsigned long long part[NV * 4];
   for (int i = threadIdx.x; i < NV * 4; i += blockDim.x) part[i] = 0;
   __syncthreads();
@@ -860,6 +855,13 @@ __device__ __forceinline__ void block_acc(const E4 (&v)[NV], unsigned long long 
     }
   __syncthreads();
   for (int i = threadIdx.x; i < NV * 4; i += blockDim.x) atomicAdd(acc + i, part[i]);
+}
+// and published; acc_base is the launch's accumulator base (acc itself when
+// unbatched)
+template <int NV>
+__device__ __forceinline__ void block_acc(const E4 (&v)[NV], unsigned long long *acc,
+                                          unsigned long long *acc_base, const Publish &pub) {
+  block_sum<NV>(v, acc);
   publish_if_last(acc_base, pub);
 }
 
@@ -868,28 +870,18 @@ __device__ __forceinline__ void block_acc(const E4 (&v)[NV], unsigned long long 
 // Batched: instance y = blockIdx.y has its arrays at y n_in (inputs) and
 // y n_in / 2 (outputs), its challenge at r_b[y] and its sums at
 // acc + y acc_stride.
+// CTA bx of nbx; the sums are this thread's part of (c0, c2).
 template <bool VEC>
-__global__ void __launch_bounds__(256) round_kernel(const E4 *__restrict__ p_in,
-                                                    const E4 *__restrict__ w_in, size_t n_in,
-                                                    int fold, E4 r, E4 *__restrict__ p_out,
-                                                    E4 *__restrict__ w_out, int coeffs,
-                                                    unsigned long long *acc, Publish pub,
-                                                    const E4 *__restrict__ r_b,
-                                                    size_t acc_stride) {
-  pdl_wait();
-  p_in += blockIdx.y * n_in;
-  w_in += blockIdx.y * n_in;
-  if (fold) {
-    p_out += blockIdx.y * (n_in / 2);
-    w_out += blockIdx.y * (n_in / 2);
-    if (r_b) r = r_b[blockIdx.y];
-  }
-  unsigned long long *const acc_y = acc + blockIdx.y * acc_stride;
+__device__ __forceinline__ void round_body(const E4 *__restrict__ p_in,
+                                           const E4 *__restrict__ w_in, size_t n_in, int fold,
+                                           const E4 &r, E4 *__restrict__ p_out,
+                                           E4 *__restrict__ w_out, int coeffs, unsigned bx,
+                                           unsigned nbx, E4 (&sums)[2]) {
   size_t n = fold ? n_in / 2 : n_in;
   size_t pairs = (n + 1) / 2;
-  E4 sums[2] = {kb::e_zero(), kb::e_zero()};
-  for (size_t m = (size_t)blockIdx.x * blockDim.x + threadIdx.x; m < pairs;
-       m += (size_t)gridDim.x * blockDim.x) {
+  sums[0] = sums[1] = kb::e_zero();
+  for (size_t m = (size_t)bx * blockDim.x + threadIdx.x; m < pairs;
+       m += (size_t)nbx * blockDim.x) {
     E4 p0, p1 = kb::e_zero(), w0, w1 = kb::e_zero();
     if (fold) {
       const E4 *pp = p_in + 4 * m, *ww = w_in + 4 * m;
@@ -921,19 +913,40 @@ __global__ void __launch_bounds__(256) round_kernel(const E4 *__restrict__ p_in,
       sums[1] = kb::e_add(sums[1], kb::e_mul(dw, dp));
     }
   }
-  if (coeffs) block_acc<2>(sums, acc_y, acc, pub);
+}
+template <bool VEC>
+__global__ void __launch_bounds__(256) round_kernel(const E4 *__restrict__ p_in,
+                                                    const E4 *__restrict__ w_in, size_t n_in,
+                                                    int fold, E4 r, E4 *__restrict__ p_out,
+                                                    E4 *__restrict__ w_out, int coeffs,
+                                                    unsigned long long *acc, Publish pub,
+                                                    const E4 *__restrict__ r_b,
+                                                    size_t acc_stride) {
+  pdl_wait();
+  p_in += blockIdx.y * n_in;
+  w_in += blockIdx.y * n_in;
+  if (fold) {
+    p_out += blockIdx.y * (n_in / 2);
+    w_out += blockIdx.y * (n_in / 2);
+    if (r_b) r = r_b[blockIdx.y];
+  }
+  E4 sums[2];
+  round_body<VEC>(p_in, w_in, n_in, fold, r, p_out, w_out, coeffs, blockIdx.x, gridDim.x, sums);
+  if (coeffs) block_acc<2>(sums, acc + blockIdx.y * acc_stride, acc, pub);
 }
 
+// CTAs of a round over n elements (after the fold): about four per SM at most
+static unsigned round_ctas(size_t n, int batch) {
+  const size_t g = ((n + 1) / 2 + 255) / 256, cap = ((size_t)152 * 4 + batch - 1) / batch;
+  return (unsigned)(g < cap ? (g ? g : 1) : cap);
+}
 static cudaError_t round_launch(const E4 *p_in, const E4 *w_in, size_t n_in, bool fold, E4 r,
                                 const E4 *r_b, E4 *p_out, E4 *w_out, bool coeffs,
                                 unsigned long long *acc, size_t acc_stride, int batch,
                                 cudaStream_t st, const Publish &pub) {
   if (batch < 1 || batch > 65535) return cudaErrorInvalidValue;
-  size_t n = fold ? n_in / 2 : n_in;
-  size_t pairs = (n + 1) / 2;
-  unsigned T = 256;
-  size_t g = (pairs + T - 1) / T, cap = ((size_t)152 * 4 + batch - 1) / batch;
-  dim3 grid((unsigned)(g < cap ? (g ? g : 1) : cap), (unsigned)batch);
+  const unsigned T = 256;
+  dim3 grid(round_ctas(fold ? n_in / 2 : n_in, batch), (unsigned)batch);
   const bool vec = aligned16(p_in) && aligned16(w_in) &&
                    (!fold || (aligned16(p_out) && aligned16(w_out)));
   if (vec)
@@ -1096,78 +1109,123 @@ cudaError_t row_evals_batch(const uint32_t *rows, int row_len, const uint32_t *i
 // 2^(r-1)) and wd = w^-S.  Each query adds its part of (c0, c2)
 // (prover.rs:503-536) to acc[0..8) and, at round 0, scales_i g(0, idx_i) to
 // acc[8..12), as canonical words; the host reduces them with the round pass.
-__device__ __forceinline__ void acc_add_e4(unsigned long long *acc, const E4 &v) {
-#pragma unroll
-  for (int c = 0; c < 4; c++) atomicAdd(acc + c, (unsigned long long)v.c[c]);
-}
-
-__device__ __forceinline__ void code_round_query(CodeState s, int round, E4 r_prev,
-                                                 unsigned long long *acc) {
+// One query per warp; lane 0 holds its part of c0, c2 and (round 0) the sum
+// term in v[0..2].
+__device__ __forceinline__ void code_query(const CodeState &s, int i, int round, const E4 &r_prev,
+                                           E4 (&v)[3]) {
   using namespace kb;
-  const int i = blockIdx.x;
+  const int lane = threadIdx.x & 31;
   const int lS = s.k_data - s.d;
   const int T = 1 << s.d;
   const uint32_t idx = s.idx[i];
   const uint32_t base = idx & ((1u << lS) - 1u), tb = idx >> lS;
   E4 *G = s.G + (size_t)i * T;
-  __shared__ uint32_t pw[3];
+  E4 sc = s.scales[i];
+  uint32_t ws, tw;
+  v[2] = e_zero();
   if (round == 0) {
     // w^idx, w^-(idx mod 2^(k_data-1)), w^-base: one exponentiation per lane
-    if (threadIdx.x < 3) {
-      uint32_t b = threadIdx.x == 0 ? s.omega : s.winv;
-      uint32_t e = threadIdx.x == 0 ? idx
-                   : threadIdx.x == 1 ? (idx & ((1u << (s.k_data - 1)) - 1u))
-                                      : base;
-      pw[threadIdx.x] = kb::pow(b, e);
+    uint32_t p = 0;
+    if (lane < 3)
+      p = kb::pow(lane == 0 ? s.omega : s.winv, lane == 0   ? idx
+                                                : lane == 1 ? idx & ((1u << (s.k_data - 1)) - 1u)
+                                                            : base);
+    ws = __shfl_sync(0xffffffffu, p, 0);
+    tw = __shfl_sync(0xffffffffu, p, 1);
+    const uint32_t B = __shfl_sync(0xffffffffu, p, 2);
+    if (lane == 0) {
+      s.ws[i] = ws;
+      s.tw[i] = tw;
+      s.B[i] = B;
+      v[2] = e_mul(sc, G[tb]);
     }
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    E4 sc = s.scales[i];
-    s.ws[i] = pw[0];
-    s.tw[i] = pw[1];
-    s.B[i] = pw[2];
-    acc_add_e4(acc + 8, e_mul(sc, G[tb]));
   } else {
     const int half = T >> round;
     const uint32_t B = s.B[i];
-    for (int t = threadIdx.x; t < half; t += blockDim.x) {
-      uint32_t tw = mul(B, s.wd[(t << (round - 1)) & (T - 1)]);
+    ws = s.ws[i];
+    tw = s.tw[i];
+    for (int t = lane; t < half; t += 32) {
+      const uint32_t wt = mul(B, s.wd[(t << (round - 1)) & (T - 1)]);
       E4 glo = G[t], ghi = G[t + half];
       E4 even = e_scale(e_add(glo, ghi), s.two_inv);
-      E4 odd = e_scale(e_sub(glo, ghi), mul(s.two_inv, tw));
+      E4 odd = e_scale(e_sub(glo, ghi), mul(s.two_inv, wt));
       G[t] = e_add(even, e_mul(r_prev, e_sub(odd, even)));
     }
-    __syncthreads();
-    if (threadIdx.x != 0) return;
     // the updates after round r-1 (prover.rs:542-553)
-    uint32_t ws = s.ws[i], tw = s.tw[i];
     E4 f = e_add(e_one(), e_mul(r_prev, e_add(e_neg(e_one()), e_from(ws))));
-    s.scales[i] = e_mul(s.scales[i], f);
+    sc = e_mul(sc, f);
     ws = mul(ws, ws);
     tw = mul(tw, tw);
     if ((idx >> (s.k_data - round - 1)) & 1u) tw = neg(tw);
-    s.ws[i] = ws;
-    s.tw[i] = tw;
-    s.B[i] = mul(B, B);
+    __syncwarp();  // G is folded, and every lane has read the old state
+    if (lane == 0) {
+      s.scales[i] = sc;
+      s.ws[i] = ws;
+      s.tw[i] = tw;
+      s.B[i] = mul(B, B);
+    }
   }
-  const E4 sc = s.scales[i];
-  const uint32_t ws = s.ws[i], tw = s.tw[i];
   const int hlf = (T >> round) / 2;
   const uint32_t tl = tb & (uint32_t)(hlf - 1);
   E4 glo = G[tl], ghi = G[tl + hlf];
   E4 even = e_scale(e_add(glo, ghi), s.two_inv);
   E4 odd = e_scale(e_scale(e_sub(glo, ghi), s.two_inv), tw);
-  acc_add_e4(acc, e_mul(sc, even));
-  uint32_t wt = sub(dbl(ws), ONE);
-  acc_add_e4(acc + 4, e_scale(e_mul(sc, e_sub(e_dbl(odd), even)), wt));
+  v[0] = e_mul(sc, even);
+  const uint32_t wt = sub(dbl(ws), ONE);
+  v[1] = e_scale(e_mul(sc, e_sub(e_dbl(odd), even)), wt);
 }
 
-__global__ void __launch_bounds__(32) code_round_kernel(CodeState s, int round, E4 r_prev,
-                                                        unsigned long long *acc, Publish pub) {
+// CTA bx: eight queries, summed in shared memory when they belong to one
+// instance
+__device__ __forceinline__ void code_cta(const CodeState &s, int round, E4 r_prev, unsigned bx,
+                                         unsigned long long *acc) {
+  __shared__ unsigned long long part[12];
+  if (threadIdx.x < 12) part[threadIdx.x] = 0;
+  __syncthreads();
+  const int q0 = 8 * (int)bx, i = q0 + (int)(threadIdx.x >> 5);
+  const int words = round == 0 ? 12 : 8;
+  const int b0 = s.inst ? s.inst[q0] : 0;
+  const bool one = !s.inst || s.inst[q0 + 7 < s.n ? q0 + 7 : s.n - 1] == b0;
+  if (i < s.n) {
+    const int b = s.inst ? s.inst[i] : 0;
+    if (s.r_b && round > 0) r_prev = s.r_b[b];
+    E4 v[3];
+    code_query(s, i, round, r_prev, v);
+    unsigned long long *to = one ? part : acc + (size_t)b * s.acc_stride;
+    if ((threadIdx.x & 31) == 0)
+      for (int c = 0; c < words; c++) atomicAdd(to + c, (unsigned long long)v[c >> 2].c[c & 3]);
+  }
+  __syncthreads();
+  if (one && (int)threadIdx.x < words)
+    atomicAdd(acc + (size_t)b0 * s.acc_stride + threadIdx.x, part[threadIdx.x]);
+}
+
+__global__ void __launch_bounds__(256) code_round_kernel(CodeState s, int round, E4 r_prev,
+                                                         unsigned long long *acc, Publish pub) {
   pdl_wait();
-  const int b = s.inst ? s.inst[blockIdx.x] : 0;
-  if (s.r_b && round > 0) r_prev = s.r_b[b];
-  code_round_query(s, round, r_prev, acc + (size_t)b * s.acc_stride);
+  code_cta(s, round, r_prev, blockIdx.x, acc);
+  publish_if_last(acc, pub);
+}
+
+// The expression's pass of a round and the code's in one launch: the first
+// `ctas` CTAs are round_kernel's, the others code_round_kernel's.  The passes
+// are independent, and at the sizes of most proofs each lasts little longer
+// than a launch (a k = 12 proof, four such rounds: 400 us in two launches
+// each, 387 us in one).
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+    round_code_kernel(const E4 *__restrict__ p_in, const E4 *__restrict__ w_in, size_t n_in,
+                      int fold, E4 r, E4 *__restrict__ p_out, E4 *__restrict__ w_out,
+                      unsigned ctas, CodeState s, int round, E4 r_prev, unsigned long long *acc,
+                      Publish pub) {
+  pdl_wait();
+  if (blockIdx.x < ctas) {
+    E4 sums[2];
+    round_body<VEC>(p_in, w_in, n_in, fold, r, p_out, w_out, 1, blockIdx.x, ctas, sums);
+    block_sum<2>(sums, acc);
+  } else {
+    code_cta(s, round, r_prev, blockIdx.x - ctas, acc);
+  }
   publish_if_last(acc, pub);
 }
 
@@ -1189,7 +1247,27 @@ cudaError_t code_round(const CodeState &s, int round, E4 r_prev, unsigned long l
   if (s.n == 0) return cudaSuccess;
   if (s.d < 1 || s.d > 8 || s.k_data < s.d || s.k_data > 30 || round < 0 || round >= s.d)
     return cudaErrorInvalidValue;
-  launch(code_round_kernel, s.n, 32, 0, st, s, round, r_prev, acc, pub);
+  launch(code_round_kernel, (s.n + 7) / 8, 256, 0, st, s, round, r_prev, acc, pub);
+  count_launches(1);
+  return cudaGetLastError();
+}
+
+cudaError_t sumcheck_round_code(const E4 *p_in, const E4 *w_in, size_t n_in, bool fold, E4 r,
+                                E4 *p_out, E4 *w_out, const CodeState &s, int round, E4 r_prev,
+                                unsigned long long *acc, cudaStream_t st, const Publish &pub) {
+  if (s.n < 1 || s.d < 1 || s.d > 8 || s.k_data < s.d || s.k_data > 30 || round < 0 ||
+      round >= s.d || s.inst)
+    return cudaErrorInvalidValue;
+  const unsigned ctas = round_ctas(fold ? n_in / 2 : n_in, 1);
+  const unsigned grid = ctas + (unsigned)(s.n + 7) / 8;
+  const bool vec = aligned16(p_in) && aligned16(w_in) &&
+                   (!fold || (aligned16(p_out) && aligned16(w_out)));
+  if (vec)
+    launch(round_code_kernel<true>, grid, 256, 0, st, p_in, w_in, n_in, fold ? 1 : 0, r, p_out,
+           w_out, ctas, s, round, r_prev, acc, pub);
+  else
+    launch(round_code_kernel<false>, grid, 256, 0, st, p_in, w_in, n_in, fold ? 1 : 0, r, p_out,
+           w_out, ctas, s, round, r_prev, acc, pub);
   count_launches(1);
   return cudaGetLastError();
 }
