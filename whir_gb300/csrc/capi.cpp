@@ -284,14 +284,18 @@ int whir_compress_hi(whir_ctx *ctx, const uint32_t *poly, int k, const uint32_t 
   need(kz >= 0 && kz <= k && k - kz <= 8, "compress_hi keeps at most 8 variables");
   whir::gpu::Point z = point_in(point, kz);
   int ks = k - kz;
-  int s_lo = kz < 10 ? kz : 10;
-  ctx->eq.reserve(sizeof(E4) * (((size_t)1 << s_lo) + ((size_t)1 << (kz - s_lo))));
-  E4 *lo = ctx->eq.as<E4>(), *hi = lo + ((size_t)1 << s_lo);
   cudaStream_t st = ctx->ctx.stream();
-  whir::cuda_check(whir::gpu::eq_split(z, s_lo, kb::e_one(), lo, hi, st), "eq_split");
   size_t words = (size_t)4 << ks;
   unsigned long long *a = acc_buf(ctx, words);
-  whir::cuda_check(whir::gpu::compress_hi(poly, k, ks, lo, s_lo, hi, a, st), "compress_hi");
+  if (k <= 28) {
+    whir::cuda_check(whir::gpu::compress_hi_point(poly, k, z, a, st), "compress_hi");
+  } else {  // its CTAs' high tables would outgrow shared memory
+    int s_lo = kz < 10 ? kz : 10;
+    ctx->eq.reserve(sizeof(E4) * (((size_t)1 << s_lo) + ((size_t)1 << (kz - s_lo))));
+    E4 *lo = ctx->eq.as<E4>(), *hi = lo + ((size_t)1 << s_lo);
+    whir::cuda_check(whir::gpu::eq_split(z, s_lo, kb::e_one(), lo, hi, st), "eq_split");
+    whir::cuda_check(whir::gpu::compress_hi(poly, k, ks, lo, s_lo, hi, a, st), "compress_hi");
+  }
   read_acc(ctx, a, words, out);
   API_END
 }
@@ -315,14 +319,20 @@ int whir_eval_ext(whir_ctx *ctx, const uint32_t *poly, int k, const uint32_t *po
   need(ctx && poly && out, "null argument");
   need(k >= 0 && k <= 30, "bad k");
   whir::gpu::Point z = point_in(point, k);
-  int s_lo = k < 10 ? k : 10;
-  ctx->eq.reserve(sizeof(E4) * (((size_t)1 << s_lo) + ((size_t)1 << (k - s_lo))));
-  E4 *lo = ctx->eq.as<E4>(), *hi = lo + ((size_t)1 << s_lo);
   cudaStream_t st = ctx->ctx.stream();
-  whir::cuda_check(whir::gpu::eq_split(z, s_lo, kb::e_one(), lo, hi, st), "eq_split");
   unsigned long long *a = acc_buf(ctx, 4);
-  whir::cuda_check(whir::gpu::eval_ext(reinterpret_cast<const E4 *>(poly), k, lo, s_lo, hi, a, st),
-                   "eval_ext");
+  if (k <= 26) {
+    whir::cuda_check(whir::gpu::eval_ext_point(reinterpret_cast<const E4 *>(poly), z, a, st),
+                     "eval_ext");
+  } else {  // its CTAs' high tables would outgrow shared memory
+    int s_lo = 10;
+    ctx->eq.reserve(sizeof(E4) * (((size_t)1 << s_lo) + ((size_t)1 << (k - s_lo))));
+    E4 *lo = ctx->eq.as<E4>(), *hi = lo + ((size_t)1 << s_lo);
+    whir::cuda_check(whir::gpu::eq_split(z, s_lo, kb::e_one(), lo, hi, st), "eq_split");
+    whir::cuda_check(
+        whir::gpu::eval_ext(reinterpret_cast<const E4 *>(poly), k, lo, s_lo, hi, a, st),
+        "eval_ext");
+  }
   read_acc(ctx, a, 4, out);
   API_END
 }
@@ -361,31 +371,39 @@ int whir_sumcheck_fold(whir_ctx *ctx, const uint32_t *poly, const uint32_t *weig
   API_END
 }
 
-int whir_combine_eqs(whir_ctx *ctx, uint32_t *weights, int k, const uint32_t *points, int n,
+int whir_combine_eqs(whir_ctx *ctx, uint32_t *weights, int k, const uint32_t *points_in, int n,
                      const uint32_t alpha[4]) {
   API_BEGIN
-  need(ctx && weights && alpha && (points || !n) && n >= 0, "bad argument");
+  need(ctx && weights && alpha && (points_in || !n) && n >= 0, "bad argument");
   need(k >= 0 && k <= 24, "bad k");
   if (n == 0) return WHIR_OK;
   E4 a = ext_in(alpha), s = kb::e_one();
-  int sl = k / 2;
-  size_t per = ((size_t)1 << sl) + ((size_t)1 << (k - sl));
-  ctx->eq.reserve(sizeof(E4) * per * n);
+  const int sl = k / 2, N = whir::gpu::EqArgs::N;
+  const size_t per = ((size_t)1 << sl) + ((size_t)1 << (k - sl));
+  const bool points = whir::gpu::add_eq_by_points(k, std::min(n, N));
+  if (!points) ctx->eq.reserve(sizeof(E4) * per * n);
   cudaStream_t st = ctx->ctx.stream();
-  whir::gpu::EqArgs q;  // the tables of up to EqArgs::N points per launch
-  for (int t0 = 0; t0 < n; t0 += whir::gpu::EqArgs::N) {
-    const int m = std::min(n - t0, (int)whir::gpu::EqArgs::N);
-    for (int t = 0; t < m; t++) {
-      const whir::gpu::Point z = point_in(points + (size_t)4 * k * (t0 + t), k);
-      std::copy(z.z, z.z + k, q.z + t * whir::gpu::EqArgs::K);
-      q.scale[t] = s;
-      s = kb::e_mul(s, a);
+  E4 *w = reinterpret_cast<E4 *>(weights);
+  whir::gpu::EqArgs q;  // up to N points per launch
+  for (int pass = 0; pass < 2; pass++) {  // every point is checked before w is touched
+    s = kb::e_one();
+    for (int t0 = 0; t0 < n; t0 += N) {
+      const int m = std::min(n - t0, N);
+      for (int t = 0; t < m; t++) {
+        const whir::gpu::Point z = point_in(points_in + (size_t)4 * k * (t0 + t), k);
+        std::copy(z.z, z.z + k, q.z + t * whir::gpu::EqArgs::K);
+        q.scale[t] = s;
+        s = kb::e_mul(s, a);
+      }
+      if (pass == 0) continue;
+      if (points)
+        whir::cuda_check(whir::gpu::add_eq_points(w, k, q, m, st), "add_eq");
+      else
+        whir::cuda_check(
+            whir::gpu::eq_tables_val(q, m, k, sl, ctx->eq.as<E4>() + per * t0, st), "eq_tables");
     }
-    whir::cuda_check(whir::gpu::eq_tables_val(q, m, k, sl, ctx->eq.as<E4>() + per * t0, st),
-                     "eq_tables");
   }
-  whir::cuda_check(whir::gpu::add_eq(reinterpret_cast<E4 *>(weights), k, ctx->eq.as<E4>(), n, st),
-                   "add_eq");
+  if (!points) whir::cuda_check(whir::gpu::add_eq(w, k, ctx->eq.as<E4>(), n, st), "add_eq");
   ctx->ctx.sync();
   API_END
 }

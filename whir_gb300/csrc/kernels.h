@@ -137,6 +137,11 @@ cudaError_t eq_full(const Point &z, kb::E4 scale, kb::E4 *out, kb::E4 *tmp, cuda
 cudaError_t compress_hi(const uint32_t *poly, int k, int ks, const kb::E4 *eq_lo, int s_lo,
                         const kb::E4 *eq_hi, unsigned long long *acc, cudaStream_t st,
                         const Publish &pub = Publish());
+// the same with the tables formed by the kernel: z holds the k - ks fixed
+// variables
+cudaError_t compress_hi_point(const uint32_t *poly, int k, const Point &z,
+                              unsigned long long *acc, cudaStream_t st,
+                              const Publish &pub = Publish());
 // SplitEq::compress_lo_into (eq.rs:491-539): out[i] = sum_j eq(rs)[j] * P[i*2^ks + j]
 cudaError_t compress_lo(const uint32_t *poly, int k, const Point &rs, kb::E4 *out,
                         cudaStream_t st);
@@ -144,6 +149,10 @@ cudaError_t compress_lo(const uint32_t *poly, int k, const Point &rs, kb::E4 *ou
 // stored back to back (lo0, hi0, lo1, hi1, ...), s = k / 2, each lo 2^s and
 // hi 2^(k-s) entries.
 cudaError_t add_eq(kb::E4 *w, int k, const kb::E4 *tables, int n_tables, cudaStream_t st);
+// w[i] += sum_t scale_t eq(z_t)[i] for n <= EqArgs::N points of k coordinates,
+// the tables formed by the kernel; add_eq_by_points: the sizes it is for
+cudaError_t add_eq_points(kb::E4 *w, int k, const EqArgs &a, int n, cudaStream_t st);
+bool add_eq_by_points(int k, int n);
 // w[i] += sum_t scale_t * var_t^i  (pow::combine_pows(_scaled), combine.rs:408-468);
 // tab: add_pows_scratch_words(k, n) words for the split power tables
 size_t add_pows_scratch_words(int k, int n);
@@ -168,6 +177,9 @@ cudaError_t sumcheck_round(const kb::E4 *p_in, const kb::E4 *w_in, size_t n_in, 
 cudaError_t eval_ext(const kb::E4 *poly, int k, const kb::E4 *eq_lo, int s_lo,
                      const kb::E4 *eq_hi, unsigned long long *acc, cudaStream_t st,
                      const Publish &pub = Publish());
+// the same with the tables formed by the kernel (z.k variables)
+cudaError_t eval_ext_point(const kb::E4 *poly, const Point &z, unsigned long long *acc,
+                           cudaStream_t st, const Publish &pub = Publish());
 // <a, b> of two extension arrays of n elements -> acc u64[4] (debug checks)
 cudaError_t dot_ext(const kb::E4 *a, const kb::E4 *b, size_t n, unsigned long long *acc,
                     cudaStream_t st, const Publish &pub = Publish());

@@ -682,15 +682,13 @@ struct Prover::Impl {
   void svo_claim(SvoClaim &c, const uint32_t *poly_dev, int kp, const E4 *point) {
     c.k = kp;
     c.point.assign(point, point + kp);
-    int nz = kp - ks;
-    int s_lo = std::min(8, nz);  // 2^(nz-8) CTAs: enough loads in flight
-    E4 *lo = eqbuf.as<E4>(), *hi = lo + ((size_t)1 << s_lo);
-    make_eq_tables({point + ks}, nz, {e_one()}, s_lo, lo);
+    gpu::Point z;
+    z.k = kp - ks;
+    std::copy(point + ks, point + kp, z.z);
     size_t na = (size_t)4 << ks;
     unsigned long long *a = acc.as<unsigned long long>();
     ctx->prof_begin(Context::K_SUMCHECK);
-    cuda_check(gpu::compress_hi(poly_dev, kp, ks, lo, s_lo, hi, a, st(), publish((int)na)),
-               "compress_hi");
+    cuda_check(gpu::compress_hi_point(poly_dev, kp, z, a, st(), publish((int)na)), "compress_hi");
     ctx->prof_end(Context::K_SUMCHECK, 4.0 * (double)((size_t)1 << kp));
     const unsigned long long *h = published();
     wait_published();
@@ -817,9 +815,22 @@ struct Prover::Impl {
     return r;
   }
 
+  static void fill_eq_args(gpu::EqArgs &a, const std::vector<std::vector<E4>> &pts,
+                           const std::vector<E4> &scales) {
+    for (size_t t = 0; t < pts.size(); t++) {
+      std::copy(pts[t].begin(), pts[t].end(), a.z + t * gpu::EqArgs::K);
+      a.scale[t] = scales[t];
+    }
+  }
   // w[off .. off + 2^kt) += eq(point) * scale for several points sharing the range
   void add_eqs(E4 *w, int kt, const std::vector<std::vector<E4>> &pts, const std::vector<E4> &scales) {
     if (pts.empty()) return;
+    if (gpu::add_eq_by_points(kt, (int)pts.size())) {
+      gpu::EqArgs a;
+      fill_eq_args(a, pts, scales);
+      cuda_check(gpu::add_eq_points(w, kt, a, (int)pts.size(), st()), "add_eq");
+      return;
+    }
     int s = kt / 2;
     size_t per = ((size_t)1 << s) + ((size_t)1 << (kt - s));
     if (per * pts.size() * sizeof(E4) > eqbuf.bytes())
@@ -1212,11 +1223,11 @@ struct Prover::Impl {
       sync();
       return *h;
     }
-    int s_lo = std::min(10, k);
-    E4 *lo = eqbuf.as<E4>(), *hi = lo + ((size_t)1 << s_lo);
-    make_eq_tables({pt.data()}, k, {e_one()}, s_lo, lo);
+    gpu::Point z;
+    z.k = k;
+    std::copy(pt.begin(), pt.end(), z.z);
     unsigned long long *a = acc.as<unsigned long long>();
-    cuda_check(gpu::eval_ext(P(), k, lo, s_lo, hi, a, st(), publish(4)), "eval_ext");
+    cuda_check(gpu::eval_ext_point(P(), z, a, st(), publish(4)), "eval_ext");
     const unsigned long long *h = published();
     wait_published();
     return reduce_acc(h);

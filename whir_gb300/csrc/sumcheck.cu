@@ -185,6 +185,57 @@ cudaError_t eq_full(const Point &z, E4 scale, E4 *out, E4 *tmp, cudaStream_t st)
   return cudaGetLastError();
 }
 
+// ---- eq tables formed by the kernel that reads them ----
+// A reading kernel needs eq(z) over the low s variables for every thread and
+// over the rest at its own blocks only.  Formed in its CTAs (PT kernels) that
+// costs less than the launch of a table kernel, whose 1 to 1.5 us on the GPU
+// and 1.8 us on the host stood before every claim, evaluation and combination
+// of a proof (us, table kernel and reader against one kernel: a claim of 2^16
+// words and 4 kept variables 5.7/4.4, of 2^24 24.5/23.8; an evaluation over
+// 2^12 elements 5.5/3.9, over 2^20 12.2/10.9).
+
+// eq over the nv variables z[0..nv) at index b
+__device__ __forceinline__ E4 eq_at(const E4 *z, int nv, unsigned b, E4 acc) {
+  for (int i = 0; i < nv; i++) {
+    const E4 zi = z[i];
+    acc = kb::e_mul(acc, ((b >> i) & 1) ? zi : kb::e_sub(kb::e_one(), zi));
+  }
+  return acc;
+}
+__device__ __forceinline__ E4 e4_shfl_xor(const E4 &v, int o) {
+  return E4{{__shfl_xor_sync(0xffffffffu, v.c[0], o), __shfl_xor_sync(0xffffffffu, v.c[1], o),
+             __shfl_xor_sync(0xffffffffu, v.c[2], o), __shfl_xor_sync(0xffffffffu, v.c[3], o)}};
+}
+// the two factors of the low table, entry i = A[i mod 2^ab] B[i >> ab] with ab
+// = (s + 1) / 2 (s <= 10): 64 entries at ab_tab, A in its first 32, B behind
+__device__ __forceinline__ E4 eq_low(const E4 *ab_tab, int s, unsigned i) {
+  const int ab = (s + 1) / 2;
+  return kb::e_mul(ab_tab[i & ((1u << ab) - 1u)], ab_tab[32 + (i >> ab)]);
+}
+// Warps 0 and 1 form A and B, the others eq over the variables z[s..k) at this
+// CTA's blocks blockIdx.x + i gridDim.x below 2^(k - s) (hi[i]), four lanes to
+// a block.  CTAs of 256 threads; a barrier follows.
+__device__ __forceinline__ void eq_prologue(const E4 *z, int k, int s, E4 *ab_tab, E4 *hi) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ab = (s + 1) / 2;
+  if (warp < 2) {
+    const int nv = warp ? s - ab : ab;
+    if (lane < (1 << nv))
+      ab_tab[32 * warp + lane] = eq_at(z + (warp ? ab : 0), nv, lane, kb::e_one());
+  } else {
+    const size_t n = (size_t)1 << (k - s);
+    const int part = lane & 3, nv = k - s, each = (nv + 3) / 4, v0 = part * each;
+    for (size_t i0 = 0; blockIdx.x + i0 * gridDim.x < n; i0 += 48) {  // warp-uniform
+      const size_t i = i0 + 8 * (warp - 2) + (lane >> 2), b = blockIdx.x + i * gridDim.x;
+      const int take = v0 >= nv ? 0 : nv - v0 < each ? nv - v0 : each;
+      E4 f = eq_at(z + s + v0, take, (unsigned)((b < n ? b : 0) >> v0), kb::e_one());
+      f = kb::e_mul(f, e4_shfl_xor(f, 1));
+      f = kb::e_mul(f, e4_shfl_xor(f, 2));
+      if (part == 0 && b < n) hi[i] = f;
+    }
+  }
+  __syncthreads();
+}
+
 // compress_hi: rows of W = 2^ks words; row h = h_lo + 2^s_lo * h_hi.  A CTA
 // walks whole h_hi blocks (2^s_lo contiguous rows); thread t always sees
 // column j = t mod W, so it keeps one inner sum (over h_lo, weighted by
@@ -210,8 +261,30 @@ __device__ __forceinline__ void ch_accumulate4(E4 &inner, const E4 *lo, int ks, 
   for (int c = 0; c < 4; c++) part4.c[c] = kb::reduce_wide(s4[c]);
   inner = kb::e_add(inner, part4);
 }
+// PT: the tables are eq(z) (z.k = k - ks variables), formed here; else read
+// from eq_lo and eq_hi.  Shared memory: lo, the column sums, and with PT the
+// low table's factors and this CTA's high entries.
+template <bool PT>
+__device__ __forceinline__ const E4 *ch_begin(unsigned char *smraw, const Point &z, int k, int ks,
+                                              const E4 *eq_lo, int s_lo) {
+  E4 *lo = reinterpret_cast<E4 *>(smraw);
+  unsigned long long *part = reinterpret_cast<unsigned long long *>(lo + ((size_t)1 << s_lo));
+  const int W = 1 << ks;
+  E4 *ab = reinterpret_cast<E4 *>(part + 4 * W), *hi = ab + 64;
+  for (int i = threadIdx.x; i < W * 4; i += CH_T) part[i] = 0;
+  if constexpr (PT) {
+    eq_prologue(z.z, k - ks, s_lo, ab, hi);
+    for (int i = threadIdx.x; i < (1 << s_lo); i += CH_T) lo[i] = eq_low(ab, s_lo, i);
+  } else {
+    for (int i = threadIdx.x; i < (1 << s_lo); i += CH_T) lo[i] = eq_lo[i];
+  }
+  __syncthreads();
+  return hi;
+}
+template <bool PT>
 __global__ void __launch_bounds__(CH_T, 4) compress_hi_kernel(const uint32_t *__restrict__ poly,
                                                               int k, int ks,
+                                                              const __grid_constant__ Point z,
                                                               const E4 *__restrict__ eq_lo,
                                                               int s_lo,
                                                               const E4 *__restrict__ eq_hi,
@@ -223,13 +296,12 @@ __global__ void __launch_bounds__(CH_T, 4) compress_hi_kernel(const uint32_t *__
   eq_lo += blockIdx.y * sd.tab;
   eq_hi += blockIdx.y * sd.tab;
   unsigned long long *const acc_y = acc + blockIdx.y * sd.acc;
-  E4 *lo = reinterpret_cast<E4 *>(smraw);
-  unsigned long long *part = reinterpret_cast<unsigned long long *>(lo + ((size_t)1 << s_lo));
+  const E4 *own_hi = ch_begin<PT>(smraw, z, k, ks, eq_lo, s_lo);
+  const E4 *lo = reinterpret_cast<const E4 *>(smraw);
+  unsigned long long *part =
+      reinterpret_cast<unsigned long long *>(smraw + (sizeof(E4) << s_lo));
   const int W = 1 << ks;
   const int tid = threadIdx.x;
-  for (int i = tid; i < (1 << s_lo); i += CH_T) lo[i] = eq_lo[i];
-  for (int i = tid; i < W * 4; i += CH_T) part[i] = 0;
-  __syncthreads();
   const size_t block_words = (size_t)W << s_lo;
   const size_t n_hi = (size_t)1 << (k - ks - s_lo);
   E4 outer = kb::e_zero();
@@ -255,7 +327,7 @@ __global__ void __launch_bounds__(CH_T, 4) compress_hi_kernel(const uint32_t *__
     }
     for (; e < block_words; e += CH_T)
       inner = kb::e_add(inner, kb::e_scale(lo[e >> ks], __ldg(base + e)));
-    outer = kb::e_add(outer, kb::e_mul(inner, eq_hi[hh]));
+    outer = kb::e_add(outer, kb::e_mul(inner, PT ? *own_hi++ : eq_hi[hh]));
   }
   // lanes of a warp that share a column add their sums by shuffles first
   // (modular adds of canonical words), so the shared atomics below see one
@@ -284,22 +356,23 @@ constexpr uint32_t CH_FOLD = (uint32_t)((1ull << 32) % kb::P);
 __device__ __forceinline__ unsigned long long ch_fold(unsigned long long x) {
   return (unsigned long long)(uint32_t)(x >> 32) * CH_FOLD + (uint32_t)x;  // < 2^57 + 2^32
 }
+template <bool PT>
 __global__ void __launch_bounds__(CH_T, 3) compress_hi_pipe_kernel(
-    const uint32_t *__restrict__ poly, int k, int ks, const E4 *__restrict__ eq_lo, int s_lo,
-    const E4 *__restrict__ eq_hi, unsigned long long *acc, Publish pub, HiStrides sd) {
+    const uint32_t *__restrict__ poly, int k, int ks, const __grid_constant__ Point z,
+    const E4 *__restrict__ eq_lo, int s_lo, const E4 *__restrict__ eq_hi,
+    unsigned long long *acc, Publish pub, HiStrides sd) {
   pdl_wait();
   extern __shared__ unsigned char smraw[];
   poly += blockIdx.y * sd.poly;
   eq_lo += blockIdx.y * sd.tab;
   eq_hi += blockIdx.y * sd.tab;
   unsigned long long *const acc_y = acc + blockIdx.y * sd.acc;
-  E4 *lo = reinterpret_cast<E4 *>(smraw);
-  unsigned long long *part = reinterpret_cast<unsigned long long *>(lo + ((size_t)1 << s_lo));
+  const E4 *own_hi = ch_begin<PT>(smraw, z, k, ks, eq_lo, s_lo);
+  const E4 *lo = reinterpret_cast<const E4 *>(smraw);
+  unsigned long long *part =
+      reinterpret_cast<unsigned long long *>(smraw + (sizeof(E4) << s_lo));
   const int W = 1 << ks;
   const int tid = threadIdx.x;
-  for (int i = tid; i < (1 << s_lo); i += CH_T) lo[i] = eq_lo[i];
-  for (int i = tid; i < W * 4; i += CH_T) part[i] = 0;
-  __syncthreads();
   const uint32_t step_rows = CH_T >> ks;
   const size_t n_hi = (size_t)1 << (k - ks - s_lo);
   const E4 *lrow = lo + (tid >> ks);
@@ -311,7 +384,7 @@ __global__ void __launch_bounds__(CH_T, 3) compress_hi_pipe_kernel(
     const uint32_t *b = poly + hh * (size_t)(16 * CH_T) + tid;
 #pragma unroll
     for (int q = 0; q < 16; q++) xa[q] = __ldcs(b + q * CH_T);
-    ha = eq_hi[hh];
+    ha = PT ? *own_hi++ : eq_hi[hh];
   }
   for (; hh < n_hi; hh += gridDim.x) {
     uint32_t xb[16];
@@ -321,7 +394,7 @@ __global__ void __launch_bounds__(CH_T, 3) compress_hi_pipe_kernel(
       const uint32_t *b = poly + nx * (size_t)(16 * CH_T) + tid;
 #pragma unroll
       for (int q = 0; q < 16; q++) xb[q] = __ldcs(b + q * CH_T);
-      hb = eq_hi[nx];
+      hb = PT ? *own_hi++ : eq_hi[nx];
     }
     unsigned long long a4[4] = {0, 0, 0, 0};
 #pragma unroll
@@ -363,25 +436,53 @@ cudaError_t compress_hi(const uint32_t *poly, int k, int ks, const E4 *eq_lo, in
   return compress_hi_batch(poly, k, ks, eq_lo, s_lo, eq_hi, acc, 1, HiStrides(), st, pub);
 }
 
-cudaError_t compress_hi_batch(const uint32_t *poly, int k, int ks, const E4 *eq_lo, int s_lo,
-                              const E4 *eq_hi, unsigned long long *acc, int batch,
-                              const HiStrides &sd, cudaStream_t st, const Publish &pub) {
+// z: PT (its own tables), one instance; else the tables at eq_lo and eq_hi
+static cudaError_t compress_hi_launch(const uint32_t *poly, int k, int ks, const Point *z,
+                                      const E4 *eq_lo, int s_lo, const E4 *eq_hi,
+                                      unsigned long long *acc, int batch, const HiStrides &sd,
+                                      cudaStream_t st, const Publish &pub) {
   if ((1 << ks) > CH_T || k < ks + s_lo || batch < 1 || batch > 65535)
     return cudaErrorInvalidValue;
   size_t n_hi = (size_t)1 << (k - ks - s_lo);
   // about four (three) CTAs per SM over all instances
-  const size_t per4 = ((size_t)152 * 4 + batch - 1) / batch, per3 = ((size_t)152 * 3 + batch - 1) / batch;
-  dim3 grid((unsigned)(n_hi < per4 ? n_hi : per4), (unsigned)batch);
+  const bool pipe = ((size_t)1 << (ks + s_lo)) == 16 * (size_t)CH_T;
+  const size_t per = ((size_t)152 * (pipe ? 3 : 4) + batch - 1) / batch;
+  dim3 grid((unsigned)(n_hi < per ? n_hi : per), (unsigned)batch);
   size_t smem = ((size_t)1 << s_lo) * sizeof(E4) + ((size_t)4 << ks) * 8;
-  if (((size_t)1 << (ks + s_lo)) == 16 * (size_t)CH_T) {
-    grid.x = (unsigned)(n_hi < per3 ? n_hi : per3);
-    launch(compress_hi_pipe_kernel, grid, CH_T, smem, st, poly, k, ks, eq_lo, s_lo, eq_hi, acc,
-           pub, sd);
+  if (z) {
+    smem += sizeof(E4) * (64 + (n_hi + grid.x - 1) / grid.x);
+    if (s_lo > 10 || z->k != k - ks || batch != 1 || smem > 48 * 1024)
+      return cudaErrorInvalidValue;
+    if (pipe)
+      launch(compress_hi_pipe_kernel<true>, grid, CH_T, smem, st, poly, k, ks, *z, eq_lo, s_lo,
+             eq_hi, acc, pub, sd);
+    else
+      launch(compress_hi_kernel<true>, grid, CH_T, smem, st, poly, k, ks, *z, eq_lo, s_lo, eq_hi,
+             acc, pub, sd);
+  } else if (pipe) {
+    launch(compress_hi_pipe_kernel<false>, grid, CH_T, smem, st, poly, k, ks, Point(), eq_lo, s_lo,
+           eq_hi, acc, pub, sd);
   } else {
-    launch(compress_hi_kernel, grid, CH_T, smem, st, poly, k, ks, eq_lo, s_lo, eq_hi, acc, pub, sd);
+    launch(compress_hi_kernel<false>, grid, CH_T, smem, st, poly, k, ks, Point(), eq_lo, s_lo,
+           eq_hi, acc, pub, sd);
   }
   count_launches(1);
   return cudaGetLastError();
+}
+
+cudaError_t compress_hi_batch(const uint32_t *poly, int k, int ks, const E4 *eq_lo, int s_lo,
+                              const E4 *eq_hi, unsigned long long *acc, int batch,
+                              const HiStrides &sd, cudaStream_t st, const Publish &pub) {
+  return compress_hi_launch(poly, k, ks, nullptr, eq_lo, s_lo, eq_hi, acc, batch, sd, st, pub);
+}
+
+cudaError_t compress_hi_point(const uint32_t *poly, int k, const Point &z,
+                              unsigned long long *acc, cudaStream_t st, const Publish &pub) {
+  // blocks of 4096 words where the polynomial has them (the pipelined kernel);
+  // shorter ones otherwise, so that a small polynomial still has several CTAs
+  const int ks = k - z.k;
+  const int s_lo = ks >= 2 && k >= 12 ? 12 - ks : z.k < 8 ? z.k : 8;
+  return compress_hi_launch(poly, k, ks, &z, nullptr, s_lo, nullptr, acc, 1, HiStrides(), st, pub);
 }
 
 // compress_lo: out[i] = sum_j eq(rs)[j] * P[i * 2^ks + j].  Batched:
@@ -494,6 +595,60 @@ cudaError_t add_eq_batch(E4 *w, int k, const E4 *tables, int n_tables, int batch
 
 cudaError_t add_eq(E4 *w, int k, const E4 *tables, int n_tables, cudaStream_t st) {
   return add_eq_batch(w, k, tables, n_tables, 1, st);
+}
+
+// w[i] += sum_t scale_t eq(z_t)[i] for at most EqArgs::N points, the tables
+// formed here: one CTA per 256 entries, whose low 8 index bits are the
+// thread's and the others the CTA's, so that point t needs the factors A_t (4
+// bits) and B_t (4 bits, times scale_t and the CTA's bits), 32 entries that
+// warp t forms.  For arrays of few CTAs (add_eq_by_points): us, tables and
+// reader against this, n points: 2^12 entries n = 1 3.3/3.1, n = 8 6.0/5.6;
+// 2^16 n = 3 4.7/4.5, n = 8 6.9/8.3; 2^18 n = 1 5.1/4.8, n = 3 7.4/10.2, and
+// one launch less.
+template <bool VEC>
+__global__ void __launch_bounds__(256) add_eq_points_kernel(E4 *__restrict__ w, int k,
+                                                            const __grid_constant__ EqArgs a,
+                                                            int n) {
+  pdl_wait();
+  __shared__ E4 A[EqArgs::N][16], B[EqArgs::N][16];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int na = k < 4 ? k : 4, nb = k < 8 ? k - na : 4, nc = k - na - nb;
+  if (warp < n) {
+    const E4 *z = a.z + warp * EqArgs::K;
+    // the CTA's bits, four lanes to a product
+    const int each = (nc + 3) / 4, v0 = (lane & 3) * each;
+    const int take = v0 >= nc ? 0 : nc - v0 < each ? nc - v0 : each;
+    E4 c = eq_at(z + na + nb + v0, take, blockIdx.x >> v0,
+                 (lane & 3) == 0 ? a.scale[warp] : kb::e_one());
+    c = kb::e_mul(c, e4_shfl_xor(c, 1));
+    c = kb::e_mul(c, e4_shfl_xor(c, 2));
+    const int b = lane & 15;
+    if (lane < 16) {
+      if (b < (1 << na)) A[warp][b] = eq_at(z, na, b, kb::e_one());
+    } else if (b < (1 << nb)) {
+      B[warp][b] = eq_at(z + na, nb, b, c);
+    }
+  }
+  __syncthreads();
+  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >> k) return;
+  E4 x = ld_e4<VEC>(w + i);
+  for (int t = 0; t < n; t++)
+    x = kb::e_add(x, kb::e_mul(A[t][threadIdx.x & ((1 << na) - 1)], B[t][threadIdx.x >> na]));
+  st_e4<VEC>(w + i, x);
+}
+
+bool add_eq_by_points(int k, int n) {
+  return n <= EqArgs::N && k <= 18 && ((size_t)n << k) <= ((size_t)1 << 18);
+}
+cudaError_t add_eq_points(E4 *w, int k, const EqArgs &a, int n, cudaStream_t st) {
+  if (n == 0) return cudaSuccess;
+  if (n > EqArgs::N || k < 0 || k > EqArgs::K || k > 31) return cudaErrorInvalidValue;
+  const unsigned g = k <= 8 ? 1u : 1u << (k - 8);
+  if (aligned16(w)) launch(add_eq_points_kernel<true>, g, 256, 0, st, w, k, a, n);
+  else launch(add_eq_points_kernel<false>, g, 256, 0, st, w, k, a, n);
+  count_launches(1);
+  return cudaGetLastError();
 }
 
 // var_t^i = lo_t[i mod 2^s] * hi_t[i >> s]: per var, 2^s low powers then
@@ -1019,6 +1174,54 @@ cudaError_t eval_ext_batch(const E4 *poly, int k, const E4 *eq_lo, int s_lo, con
 cudaError_t eval_ext(const E4 *poly, int k, const E4 *eq_lo, int s_lo, const E4 *eq_hi,
                      unsigned long long *acc, cudaStream_t st, const Publish &pub) {
   return eval_ext_batch(poly, k, eq_lo, s_lo, eq_hi, 0, 1, acc, st, pub);
+}
+
+// The same of one instance with its tables formed here: thread t holds entries
+// t of its CTA's blocks of 256, so its own low entry is one factor at the end.
+template <bool VEC>
+__global__ void __launch_bounds__(256) eval_ext_point_kernel(const E4 *__restrict__ poly, int k,
+                                                             const __grid_constant__ Point z,
+                                                             unsigned long long *acc,
+                                                             Publish pub) {
+  pdl_wait();
+  extern __shared__ E4 ev_sm[];  // 64 factors of the low table, this CTA's high entries
+  const int s = k < 8 ? k : 8;
+  eq_prologue(z.z, k, s, ev_sm, ev_sm + 64);
+  const size_t n_hi = (size_t)1 << (k - s);
+  E4 sum = kb::e_zero();
+  if (threadIdx.x < (1 << s)) {
+    const E4 *hi = ev_sm + 64;
+    size_t hh = blockIdx.x;
+    for (; hh + 3 * (size_t)gridDim.x < n_hi; hh += 4 * (size_t)gridDim.x, hi += 4) {
+      E4 x[4];  // four loads in flight
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        x[q] = ld_e4<VEC>(poly + ((hh + q * (size_t)gridDim.x) << s) + threadIdx.x);
+#pragma unroll
+      for (int q = 0; q < 4; q++) sum = kb::e_add(sum, kb::e_mul(hi[q], x[q]));
+    }
+    for (; hh < n_hi; hh += gridDim.x)
+      sum = kb::e_add(sum, kb::e_mul(*hi++, ld_e4<VEC>(poly + (hh << s) + threadIdx.x)));
+    sum = kb::e_mul(sum, eq_low(ev_sm, s, threadIdx.x));
+  }
+  E4 v[1] = {sum};
+  block_acc<1>(v, acc, acc, pub);
+}
+
+cudaError_t eval_ext_point(const E4 *poly, const Point &z, unsigned long long *acc,
+                           cudaStream_t st, const Publish &pub) {
+  const int k = z.k;
+  if (k < 0 || k > MAX_VARS) return cudaErrorInvalidValue;
+  const size_t n_hi = k < 8 ? 1 : (size_t)1 << (k - 8);
+  const unsigned grid = (unsigned)(n_hi < 152 * 8 ? n_hi : 152 * 8);
+  const size_t smem = sizeof(E4) * (64 + (n_hi + grid - 1) / grid);
+  if (smem > 48 * 1024) return cudaErrorInvalidValue;
+  if (aligned16(poly))
+    launch(eval_ext_point_kernel<true>, grid, 256, smem, st, poly, k, z, acc, pub);
+  else
+    launch(eval_ext_point_kernel<false>, grid, 256, smem, st, poly, k, z, acc, pub);
+  count_launches(1);
+  return cudaGetLastError();
 }
 
 // <poly, weights> = sum_i poly[i] weights[i] (Expression::prod, the debug
