@@ -304,14 +304,15 @@ struct Tw8 {
 // R radix-2 DIF stages in registers (see dif_step).  LAST: the final step of
 // the transform, where the block stride q is 1, the first half-size is
 // 2^(R-1) and position 0 of every stage has twiddle 1.
-template <int C, int R, bool LAST, class TW>
+// HOIST: hold the twiddles of a thread's tasks in registers.
+template <int C, int R, bool LAST, bool HOIST = true, class TW>
 __device__ __forceinline__ void dif_step_v(uint4 *tile, const TW &tw, int rows_log, int lh) {
   constexpr int T = 1 << R, V = C / 4, LV = V == 2 ? 1 : 0;
   const int lq = LAST ? 0 : lh - (R - 1);
   const int q = 1 << lq;
   const int H = LAST ? (1 << (R - 1)) : (1 << lh);
   const int tasks = (1 << (rows_log - R)) << LV;
-  if constexpr (R == 3 && !LAST && std::is_same<TW, TwShoup>::value) {
+  if constexpr (HOIST && R == 3 && !LAST && std::is_same<TW, TwShoup>::value) {
     // every task of a thread has the same block offset j when the block's
     // task stride is a multiple of q: its 7 twiddles are loaded once
     if (((blockDim.x >> LV) & (q - 1)) == 0) {
@@ -342,6 +343,8 @@ __device__ __forceinline__ void dif_step_v(uint4 *tile, const TW &tw, int rows_l
       return;
     }
   }
+  constexpr int UNROLL = R == 3 ? 1 : 2;  // overlaps two short tasks' twiddle loads
+#pragma unroll UNROLL
   for (int task = threadIdx.x; task < tasks; task += blockDim.x) {
     const int c = task & (V - 1), rest = task >> LV;
     const int j = rest & (q - 1), blk = rest >> lq;
@@ -555,24 +558,52 @@ __device__ __forceinline__ void dif_last_v(const uint4 *tile, const TW &tw, int 
         else v[t + span] = TwShoup::submul_w(a, b, wl[hh + tl]);
       }
     }
+    // the task's rows are one sub-transform's outputs k0 + m 2^(S-3), m = the
+    // bit-reversed row
+    const uint32_t o = o0 + (uint32_t)(base >> S);
+    const uint32_t k0 = brev((uint32_t)(base & (n - 1)), S);
+    const uint32_t om = o & ix.post_mask;
+    const uint32_t e0 = om * ((o >> ix.post_shift) + (k0 << ix.post_kshift));
+    const uint32_t es = om << (S - 3 + ix.post_kshift);
+    // C = 4: their twiddles as a geometric sequence in m, two table lookups
+    // and a product per row (2^19 rows of 20 words 78.6 -> 73.6 us); at C = 8
+    // lane pairs share the lookups, and eight independent ones are faster
+    // (2^21 rows of 64 words 598 against 629 us)
+    uint32_t f = 0, g = 0;
+    if (C == 4 && tw_log) {
+      f = root_pow((e0 & tmask) << (24 - tw_log));
+      g = root_pow((es & tmask) << (24 - tw_log));
+    }
 #pragma unroll
-    for (int t = 0; t < T; t++) {
-      const int r = base + t;
-      const uint32_t o = o0 + (uint32_t)(r >> S);
-      const uint32_t k = brev((uint32_t)(r & (n - 1)), S);
-      uint4 x = v[t];
+    for (int m = 0; m < T; m++) {
+      uint4 x = v[(m & 1) << 2 | (m & 2) | (m & 4) >> 2];
       if (tw_log) {
-        const uint32_t e = (o & ix.post_mask) * ((o >> ix.post_shift) + (k << ix.post_kshift));
-        x = mul4(x, root_pow((e & tmask) << (24 - tw_log)));
+        if (C == 4) {
+          x = mul4(x, f);
+          if (m + 1 < T) f = kb::mul(f, g);
+        } else {
+          x = mul4(x, root_pow(((e0 + (uint32_t)m * es) & tmask) << (24 - tw_log)));
+        }
       }
-      out4[(o * a_out + k * b_out) * wv + v0 + c] = x;
+      out4[(o * a_out + (k0 + ((uint32_t)m << (S - 3))) * b_out) * wv + v0 + c] = x;
     }
   }
 }
 
 // MINB: CTAs per SM the registers must allow; tiles of more than 48 KB fit
-// three per SM by shared memory, so they take up to 80 registers a thread
-template <int C, int MINB>
+// three per SM by shared memory, so they take up to 80 registers a thread.
+// MODE: S mod 3 for S >= 6, 3 for S = 4 and 5, so that a kernel holds only the
+// steps of its sizes (one kernel for all spilled at 80 registers).
+// Bound by the latency of the global steps: with the S mod 3 stages first a
+// thread of S = 10 or 11 had two or four loads in flight; with radix 8 first
+// and last it has eight, and the stores of a row follow its twiddle at once.
+// 2^21 rows of 64 words from 2^16 636 -> 607 us, 2^20 of 16 from 2^18
+// 93.7 -> 86.2 us, 2^20 of 64 from 2^12 292 -> 275 us, 2^19 of 20 from
+// 200003 79.3 -> 72.0 us; sizes of one wave within 0.4 us either way.
+// HOIST (twiddles of a thread's tasks loaded once) spills at the 64 registers
+// of four CTAs (2^20 rows of 16 words 87.6 us with it), so only the three-CTA
+// tiles take it.
+template <int C, int MINB, int MODE>
 __global__ void __launch_bounds__(256, MINB) dft_tile_v2(const uint32_t *__restrict__ in,
                                                    uint32_t *__restrict__ out, int S, int lg,
                                                    uint32_t width, uint32_t rows_valid,
@@ -590,19 +621,41 @@ __global__ void __launch_bounds__(256, MINB) dft_tile_v2(const uint32_t *__restr
   const uint4 *in4 = reinterpret_cast<const uint4 *>(in);
   uint4 *out4 = reinterpret_cast<uint4 *>(out);
   const int rows_log = S + lg;
-  const int r0 = S % 3 == 0 ? 3 : S % 3;
-  if (r0 == 1)
-    dif_first_v<C, 1>(tile, aux, rows_log, S, in4, o0, wv, v0, rows_valid, a_in, b_in, pre_log,
-                         ix);
-  else if (r0 == 2)
-    dif_first_v<C, 2>(tile, aux, rows_log, S, in4, o0, wv, v0, rows_valid, a_in, b_in, pre_log,
-                         ix);
-  else
+  // Radix 8 first and last (the steps on global memory: eight loads in
+  // flight per thread), radix 8 and the remaining one to four stages between.
+  if constexpr (MODE < 3) {
     dif_first_v<C, 3>(tile, aux, rows_log, S, in4, o0, wv, v0, rows_valid, a_in, b_in, pre_log,
-                         ix);
-  __syncthreads();
-  for (int lh = S - 1 - r0; lh >= 5; lh -= 3) {
-    dif_step_v<C, 3, false>(tile, aux, rows_log, lh);
+                      ix);
+    __syncthreads();
+    int lh = S - 4;
+    if constexpr (MODE == 1) {
+      if (S >= 10) {  // four stages: 2 + 2
+        dif_step_v<C, 2, false, MINB == 3>(tile, aux, rows_log, lh);
+        __syncthreads();
+        dif_step_v<C, 2, false, MINB == 3>(tile, aux, rows_log, lh - 2);
+        __syncthreads();
+        lh -= 4;
+      } else {
+        dif_step_v<C, 1, false, MINB == 3>(tile, aux, rows_log, lh);
+        __syncthreads();
+        lh -= 1;
+      }
+    } else if constexpr (MODE == 2) {
+      dif_step_v<C, 2, false, MINB == 3>(tile, aux, rows_log, lh);
+      __syncthreads();
+      lh -= 2;
+    }
+    for (; lh >= 5; lh -= 3) {
+      dif_step_v<C, 3, false, MINB == 3>(tile, aux, rows_log, lh);
+      __syncthreads();
+    }
+  } else {
+    if (S == 4)
+      dif_first_v<C, 1>(tile, aux, rows_log, S, in4, o0, wv, v0, rows_valid, a_in, b_in, pre_log,
+                        ix);
+    else
+      dif_first_v<C, 2>(tile, aux, rows_log, S, in4, o0, wv, v0, rows_valid, a_in, b_in, pre_log,
+                        ix);
     __syncthreads();
   }
   dif_last_v<C>(tile, aux, rows_log, S, out4, o0, wv, v0, a_out, b_out, tw_log, ix);
@@ -621,14 +674,17 @@ static cudaError_t launch_tile_v(const uint32_t *in, uint32_t *out, int S, size_
   int threads = (int)(rows * (C / 4) / 8);
   threads = threads < 32 ? 32 : (threads > 256 ? 256 : threads);
   dim3 grid((unsigned)(width / C), (unsigned)(n_outer >> lg));
-  if (S >= 4 && rows * C * 4 > (48u << 10))
-    launch(dft_tile_v2<C, 3>, grid, threads, rows * C * 4, st, in, out, S, lg, (uint32_t)width,
+  if (S >= 4) {
+    // above 48 KB: sub-transforms of 2^12 rows, and of 2^11 at C = 8
+    static const decltype(&dft_tile_v2<C, 4, 0>) narrow[4] = {
+        dft_tile_v2<C, 4, 0>, dft_tile_v2<C, 4, 1>, dft_tile_v2<C, 4, 2>, dft_tile_v2<C, 4, 3>};
+    const auto kernel = rows * C * 4 <= (48u << 10) ? narrow[S < 6 ? 3 : S % 3]
+                        : S == 12                   ? dft_tile_v2<C, 3, 0>
+                                                    : dft_tile_v2<C, 3, C == 8 ? 2 : 0>;
+    launch(kernel, grid, threads, rows * C * 4, st, in, out, S, lg, (uint32_t)width,
            (uint32_t)rows_valid, (uint32_t)a_in, (uint32_t)b_in, (uint32_t)a_out,
            (uint32_t)b_out, pre_log, tw_log, ix);
-  else if (S >= 4)
-    launch(dft_tile_v2<C, 4>, grid, threads, rows * C * 4, st, in, out, S, lg, (uint32_t)width,
-           (uint32_t)rows_valid, (uint32_t)a_in, (uint32_t)b_in, (uint32_t)a_out,
-           (uint32_t)b_out, pre_log, tw_log, ix);
+  }
   else
     launch(dft_tile_v<C>, grid, threads, smem, st, in, out, S, lg, (uint32_t)width,
            (uint32_t)rows_valid, (uint32_t)a_in, (uint32_t)b_in, (uint32_t)a_out,
@@ -773,6 +829,15 @@ cudaError_t dft_batch(const uint32_t *in, size_t h_in, size_t width, int log_h, 
 
 static size_t tile_smem_max(int C) { return ((size_t)(1 << MAX_TILE_LOG) * C + (1 << MAX_TILE_LOG)) * 4; }
 
+template <int C>
+static cudaError_t set_tile_v2_smem() {
+  const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  cudaError_t e = cudaFuncSetAttribute(dft_tile_v2<C, 3, 0>, a, tile_smem_max(C));
+  if (C == 8 && e == cudaSuccess)
+    e = cudaFuncSetAttribute(dft_tile_v2<C, 3, C == 8 ? 2 : 0>, a, tile_smem_max(C));
+  return e;
+}
+
 // Once per process and device; contexts on several host threads may call it.
 cudaError_t init_device_tables() {
   static std::mutex mu;
@@ -790,10 +855,8 @@ cudaError_t init_device_tables() {
   if (e == cudaSuccess) e = cudaFuncSetAttribute(dft_tile<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_max(1));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(dft_tile_v<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_max(8));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(dft_tile_v<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_max(4));
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(dft_tile_v2<8, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_max(8));
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(dft_tile_v2<4, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_max(4));
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(dft_tile_v2<8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_max(8));
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(dft_tile_v2<4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem_max(4));
+  if (e == cudaSuccess) e = set_tile_v2_smem<8>();
+  if (e == cudaSuccess) e = set_tile_v2_smem<4>();
   if (e == cudaSuccess) done[dev] = true;
   return e;
 }
