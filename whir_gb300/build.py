@@ -21,6 +21,7 @@ LIB = os.path.join(LIBDIR, "libwhir_gb300.so")
 CU_SOURCES = ["ntt.cu", "merkle.cu", "merkle_tensor.cu", "sumcheck.cu", "noalloc.cu"]
 CPP_SOURCES = ["poseidon2_host.cpp", "p2_matrix.cpp", "transcript.cpp", "svo_host.cpp", "prover.cpp", "batch_prover.cpp", "batch.cpp", "verifier.cpp", "verify_batch.cpp", "tune.cpp",
                "capi.cpp"]
+HOST_SOURCES = ["poseidon2_host.cpp"]  # vector types: not through nvcc's front end
 GENCODE = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 
@@ -53,7 +54,7 @@ def _compile(src, verbose):
         return obj
     cmd = [nvcc(), *GENCODE, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
            "-Xcompiler", "-fvisibility=hidden", "-I", CSRC, "-I", INCLUDE, "-c", path, "-o", obj]
-    if src.endswith(".cpp"):
+    if src.endswith(".cpp") and src not in HOST_SOURCES:
         cmd[1:1] = ["-x", "cu"]
     if verbose:
         cmd.append("-Xptxas=-v")
