@@ -255,9 +255,9 @@ const Lanes16 &lanes16() {
   return t;
 }
 
-// light layer of canonical words plus the next round's constants: 64-bit
-// lanes below 36 p (rows of 2 3 1 1 in four blocks, the own one twice), folded
-// once with 2^31 = 2^24 - 1 to below 2^31 + 35 2^24 < 1.4 2^31
+// light layer of words below 1.02 p plus the next round's constants: 64-bit
+// lanes below 37 p (rows of 2 3 1 1 in four blocks, the own one twice), folded
+// once with 2^31 = 2^24 - 1 to below 2^31 + 37 2^24 < 1.4 2^31
 inline void light16(V4 *x, const D2 (*rc)[2]) {
   D2 y[4][2];
   for (int h = 0; h < 2; h++) {
@@ -316,7 +316,10 @@ void permute16(const Poseidon2Constants &c, uint32_t *st) {
   const Lanes16 &t = lanes16();
   const uint32_t mu = t.mu[0];
   V4 x[4];
-  for (int j = 0; j < 4; j++) x[j] = V4{st[j], st[4 + j], st[8 + j], st[12 + j]};
+  for (int j = 0; j < 4; j++) {
+    x[j] = V4{st[j], st[4 + j], st[8 + j], st[12 + j]};
+    x[j] = vmin(x[j], x[j] - kb::P);  // any word is below 1.02 p now
+  }
   light16(x, t.rc[0]);
   for (int r = 0; r < 4; r++) {
     for (int j = 0; j < 4; j++) x[j] = vcube(x[j], t.mu);
