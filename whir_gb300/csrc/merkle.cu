@@ -71,6 +71,11 @@ static bool leaves_on_tensor(size_t n_rows, int row_len) {
 static int leaf_lanes(size_t n_rows) {
   return n_rows <= ((size_t)1 << 10) ? 32 : n_rows <= ((size_t)1 << 13) ? 4 : 0;
 }
+// Lanes per opened path (0: one thread): 13 to 18 permutations follow one
+// another.  us, warp / quad / thread, paths of 16 words and 14 levels mixed
+// with some of 64 and 12: 128 paths 36/53/116, 1024 42/54/106, 2048 64/54/108,
+// 8192 190/71/100, 11264 -/95/98, 16384 -/122/98.
+static int path_lanes(int n) { return n <= 1024 ? 32 : n <= 10240 ? 4 : 0; }
 static bool nodes_on_tensor(size_t nodes) { return nodes >= ((size_t)1 << 17); }
 
 // One row per thread; a row of ROW = 16·c words is c permutations
@@ -229,11 +234,111 @@ __global__ void __launch_bounds__(128) verify_paths_kernel(const PathDesc *__res
   ok[i] = good ? 1 : 0;
 }
 
+// One opening per warp (LANES = 32, a state word per lane) or per four lanes
+// (word l + 4j in lane l's j-th register): the sponge and the path one after
+// the other wait for permutations only.  A warp's quads run as many
+// permutations as its longest opening; the surplus is dropped.
+__global__ void __launch_bounds__(128) verify_paths_warp(const PathDesc *__restrict__ d,
+                                                         const uint32_t *__restrict__ words,
+                                                         const uint32_t *__restrict__ roots, int n,
+                                                         uint8_t *__restrict__ ok) {
+  P2Warp<24> leaf;
+  leaf.init(g_p2_24);
+  P2Warp<16> node;
+  node.init(g_p2_16);
+  pdl_wait();
+  const int i = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+  if (i >= n) return;
+  const PathDesc pd = d[i];
+  const uint32_t *w = words + pd.off, *sib = w + pd.row_len;
+  const int lane = leaf.lane;
+  uint32_t x = 0;
+  for (int pos = 0; pos < pd.row_len; pos += 16) {
+    if (lane < 16 && pos + lane < pd.row_len) x = w[pos + lane];
+    x = leaf.permute(x);
+  }
+  uint64_t idx = pd.index;
+  for (int l = 0; l < pd.log_h; l++) {
+    const uint64_t mid = 1ull << (pd.log_h - l - 1);
+    const uint32_t s = lane < 16 ? sib[8 * l + (lane & 7)] : 0;
+    const uint32_t acc = __shfl_sync(0xffffffffu, x, lane & 7);
+    // lanes 0..7 hold the left child: the node itself or, for a right one,
+    // its sibling
+    x = lane < 16 ? ((lane < 8) == (idx < mid) ? acc : s) : 0;
+    x = node.permute(x);
+    idx &= mid - 1;
+  }
+  const bool same = lane >= 8 || x == roots[8 * (size_t)i + lane];
+  const bool good = __all_sync(0xffffffffu, same);
+  if (lane == 0) ok[i] = good ? 1 : 0;
+}
+
+__global__ void __launch_bounds__(128) verify_paths_quad(const PathDesc *__restrict__ d,
+                                                         const uint32_t *__restrict__ words,
+                                                         const uint32_t *__restrict__ roots, int n,
+                                                         uint8_t *__restrict__ ok) {
+  __shared__ uint32_t kc24[P2Quad<24>::CONSTS], kc16[P2Quad<16>::CONSTS];
+  for (int i = threadIdx.x; i < P2Quad<24>::CONSTS; i += blockDim.x) kc24[i] = __ldg(g_p2_24 + i);
+  for (int i = threadIdx.x; i < P2Quad<16>::CONSTS; i += blockDim.x) kc16[i] = __ldg(g_p2_16 + i);
+  P2Quad<24> leaf;
+  leaf.init(g_p2_24, kc24);
+  P2Quad<16> node;
+  node.init(g_p2_16, kc16);
+  __syncthreads();
+  pdl_wait();
+  const int i = blockIdx.x * (blockDim.x / 4) + (threadIdx.x >> 2), lane = leaf.l;
+  const bool live = i < n;  // a whole warp permutes together
+  PathDesc pd = {};
+  if (live) pd = d[i];
+  const uint32_t *w = words + pd.off, *sib = w + pd.row_len;
+  uint32_t x[6] = {0, 0, 0, 0, 0, 0};
+  const int row_max = (int)__reduce_max_sync(0xffffffffu, (unsigned)pd.row_len);
+  for (int pos = 0; pos < row_max; pos += 16) {
+    uint32_t y[6];
+#pragma unroll
+    for (int j = 0; j < 6; j++) {
+      y[j] = x[j];
+      if (j < 4 && pos + 4 * j + lane < pd.row_len) y[j] = w[pos + 4 * j + lane];
+    }
+    leaf.permute(y);
+#pragma unroll
+    for (int j = 0; j < 6; j++)
+      if (pos < pd.row_len) x[j] = y[j];
+  }
+  uint32_t a0 = x[0], a1 = x[1];
+  uint64_t idx = pd.index;
+  const int height = (int)__reduce_max_sync(0xffffffffu, (unsigned)pd.log_h);
+  for (int l = 0; l < height; l++) {
+    const bool on = l < pd.log_h;
+    const uint64_t mid = on ? 1ull << (pd.log_h - l - 1) : 1;
+    const bool right = idx >= mid;
+    uint32_t s0 = 0, s1 = 0;
+    if (on) {
+      s0 = sib[8 * l + lane];
+      s1 = sib[8 * l + 4 + lane];
+    }
+    uint32_t t[4] = {right ? s0 : a0, right ? s1 : a1, right ? a0 : s0, right ? a1 : s1};
+    node.permute(t);
+    if (on) {
+      a0 = t[0];
+      a1 = t[1];
+      idx &= mid - 1;
+    }
+  }
+  bool same = true;
+  if (live) same = a0 == roots[8 * (size_t)i + lane] && a1 == roots[8 * (size_t)i + 4 + lane];
+  const unsigned votes = __ballot_sync(0xffffffffu, same);
+  if (live && lane == 0) ok[i] = (votes >> (threadIdx.x & 28) & 15u) == 15u ? 1 : 0;
+}
+
 cudaError_t verify_paths(const PathDesc *d, const uint32_t *words, const uint32_t *roots, int n,
                          uint8_t *ok, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   const int T = 128;
-  launch(verify_paths_kernel, (unsigned)((n + T - 1) / T), T, 0, st, d, words, roots, n, ok);
+  const int lanes = path_lanes(n);
+  const unsigned per = lanes ? T / lanes : T;
+  launch(lanes == 32 ? verify_paths_warp : lanes == 4 ? verify_paths_quad : verify_paths_kernel,
+         ((unsigned)n + per - 1) / per, T, 0, st, d, words, roots, n, ok);
   count_launches(1);
   return cudaGetLastError();
 }
