@@ -63,26 +63,30 @@ static bool leaves_on_tensor(size_t n_rows, int row_len) {
   return n_rows >= (row_len <= 16 ? (size_t)1 << 17 : (size_t)1 << 16);
 }
 // Lanes per row of small launches (0: one thread).  A thread takes a
-// permutation's latency of 10.3 us per chunk however few the rows are, a quad
-// of lanes 4.4 us, a warp 2.1 us; the instructions grow the other way.  us,
-// warp / quad / thread: 16-word rows 2^9 3.8/6.0/11.0, 2^11 6.1/6.0/11.1, 2^12
-// 9.0/6.1/11.1, 2^13 16/7.7/11.0, 2^14 29/13/11.1; 64-word rows 2^9
-// 10/17.6/41, 2^11 19/17.7/41, 2^12 31/17.8/41, 2^13 56/24/41, 2^14 106/45/41.
+// permutation's latency of 8.5 us per chunk however few the rows are, a quad
+// of lanes 4.2 us, a warp 2.1 us; the instructions grow the other way.  us,
+// warp / quad / thread: 16-word rows 2^9 3.8/5.7/9.1, 2^11 6.1/5.7/9.1, 2^12
+// 9.0/5.8/9.1, 2^13 16/7.2/9.2, 2^14 29/11.9/9.2; 64-word rows 2^9
+// 10/16.7/32, 2^11 19/16.8/32, 2^12 31/16.8/33, 2^13 56/23/33, 2^14 106/41/33.
 static int leaf_lanes(size_t n_rows) {
   return n_rows <= ((size_t)1 << 10) ? 32 : n_rows <= ((size_t)1 << 13) ? 4 : 0;
 }
 // Lanes per opened path (0: one thread): 13 to 18 permutations follow one
 // another.  us, warp / quad / thread, paths of 16 words and 14 levels mixed
-// with some of 64 and 12: 128 paths 36/53/116, 1024 42/54/106, 2048 64/54/108,
-// 8192 190/71/100, 11264 -/95/98, 16384 -/122/98.
+// with some of 64 and 12: 128 paths 34/51/111, 1024 40/52/101, 2048 62/52/102,
+// 8192 184/68/102, 11264 -/94/102, 16384 -/118/102.
 static int path_lanes(int n) { return n <= 1024 ? 32 : n <= 10240 ? 4 : 0; }
 static bool nodes_on_tensor(size_t nodes) { return nodes >= ((size_t)1 << 17); }
 
 // One row per thread; a row of ROW = 16·c words is c permutations
 // (PaddingFreeSponge: overwrite the 16 rate lanes, permute).  Base rows are
 // 2^f words and extension rows 4·2^f, so foldings 4..6 use 16..256.
+// The bound of six CTAs lets a permutation use 64 registers: left at 40 (32 in
+// compress_level), its S-boxes and additions follow one another, which a full
+// SM hides but few rows do not (2^14 rows of 64 words 41.2 -> 32.7 us, 2^15
+// 58.5 -> 50.1, 2^16 106 -> 94, 2^17 157.2 -> 156.5; 2^15 nodes 10.3 -> 9.3).
 template <int ROW>
-__global__ void __launch_bounds__(128) hash_rows_fixed(const uint32_t *__restrict__ rows,
+__global__ void __launch_bounds__(128, 6) hash_rows_fixed(const uint32_t *__restrict__ rows,
                                                        size_t n_rows,
                                                        uint32_t *__restrict__ digests) {
   pdl_wait();
@@ -111,7 +115,7 @@ __global__ void __launch_bounds__(128) hash_rows_fixed(const uint32_t *__restric
 
 // One row per warp (p2_lanes.cuh), any row length and alignment: a lane loads
 // its word of the next chunk before this chunk's permutation.
-__global__ void __launch_bounds__(128) hash_rows_warp(const uint32_t *__restrict__ rows,
+__global__ void __launch_bounds__(128, 6) hash_rows_warp(const uint32_t *__restrict__ rows,
                                                       size_t n_rows, int row_len,
                                                       uint32_t *__restrict__ digests) {
   P2Warp<24> p;
@@ -132,7 +136,7 @@ __global__ void __launch_bounds__(128) hash_rows_warp(const uint32_t *__restrict
 }
 
 // One row per four lanes, any row length and alignment.
-__global__ void __launch_bounds__(128) hash_rows_quad(const uint32_t *__restrict__ rows,
+__global__ void __launch_bounds__(128, 6) hash_rows_quad(const uint32_t *__restrict__ rows,
                                                       size_t n_rows, int row_len,
                                                       uint32_t *__restrict__ digests) {
   __shared__ uint32_t kc[P2Quad<24>::CONSTS];
@@ -164,7 +168,7 @@ __global__ void __launch_bounds__(128) hash_rows_quad(const uint32_t *__restrict
 
 // Any row length (small foldings): the trailing partial chunk overwrites only
 // its lanes and is permuted; an empty trailing chunk is not.
-__global__ void hash_rows_generic(const uint32_t *__restrict__ rows, size_t n_rows, int row_len,
+__global__ void __launch_bounds__(128, 6) hash_rows_generic(const uint32_t *__restrict__ rows, size_t n_rows, int row_len,
                                   uint32_t *__restrict__ digests) {
   pdl_wait();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -188,7 +192,7 @@ __global__ void hash_rows_generic(const uint32_t *__restrict__ rows, size_t n_ro
 // width-16 compression per level with the sibling on the side the index's
 // bit names (halves pairing: at a level of 2m nodes, index i >= m is the
 // right child).
-__global__ void __launch_bounds__(128) verify_paths_kernel(const PathDesc *__restrict__ d,
+__global__ void __launch_bounds__(128, 6) verify_paths_kernel(const PathDesc *__restrict__ d,
                                                            const uint32_t *__restrict__ words,
                                                            const uint32_t *__restrict__ roots,
                                                            int n, uint8_t *__restrict__ ok) {
@@ -238,7 +242,7 @@ __global__ void __launch_bounds__(128) verify_paths_kernel(const PathDesc *__res
 // (word l + 4j in lane l's j-th register): the sponge and the path one after
 // the other wait for permutations only.  A warp's quads run as many
 // permutations as its longest opening; the surplus is dropped.
-__global__ void __launch_bounds__(128) verify_paths_warp(const PathDesc *__restrict__ d,
+__global__ void __launch_bounds__(128, 6) verify_paths_warp(const PathDesc *__restrict__ d,
                                                          const uint32_t *__restrict__ words,
                                                          const uint32_t *__restrict__ roots, int n,
                                                          uint8_t *__restrict__ ok) {
@@ -273,7 +277,7 @@ __global__ void __launch_bounds__(128) verify_paths_warp(const PathDesc *__restr
   if (lane == 0) ok[i] = good ? 1 : 0;
 }
 
-__global__ void __launch_bounds__(128) verify_paths_quad(const PathDesc *__restrict__ d,
+__global__ void __launch_bounds__(128, 6) verify_paths_quad(const PathDesc *__restrict__ d,
                                                          const uint32_t *__restrict__ words,
                                                          const uint32_t *__restrict__ roots, int n,
                                                          uint8_t *__restrict__ ok) {
@@ -375,7 +379,7 @@ cudaError_t hash_rows(const uint32_t *rows, size_t n_rows, int row_len, uint32_t
   return cudaGetLastError();
 }
 
-__global__ void __launch_bounds__(128) compress_level(const uint32_t *__restrict__ src,
+__global__ void __launch_bounds__(128, 6) compress_level(const uint32_t *__restrict__ src,
                                                       uint32_t *__restrict__ dst, size_t half) {
   pdl_wait();
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
