@@ -49,16 +49,17 @@ cudaError_t init_poseidon2_tables() {
 }
 
 // Where the tensor-core kernels (merkle_tensor.cu) take over.  Their tiles
-// are 128 rows and 608 of them fill the GPU; a tile takes 9.2 us per width-24
-// permutation alone on its SM and 16.5 us among four, so launches of few
-// tiles per SM gain nothing over one thread per row.  Measured, tensor
-// against thread, us: 16-word rows 2^15 17.5/16.3, 2^16 23.6/28.8, 2^17
-// 38.6/45.4, 2^22 909/1163; 64-word rows 2^15 55.6/58.9, 2^16 74.5/107, 2^22
-// 3 550/4 912; nodes 2^16 17.8/18.8, 2^17 27.8/29.0, 2^21 330/381.  A tensor
-// launch takes an SM's whole register file and thread-per-row launches of
-// these sizes do not, so where several streams share the GPU the lines lie
-// one size above the break-even alone (32 jobs of 2^14..2^20 evaluations on
-// 8 streams: 8.95 ms, 9.1 ms with the lines one size lower).
+// are 128 rows and 608 of them (760 of nodes) fill the GPU; a tile takes 9.2 us
+// per width-24 permutation alone on its SM and 16.5 us among four, so launches
+// of few tiles per SM gain nothing over one thread per row.  Measured, tensor
+// against thread, us: 16-word rows 2^15 16.9/14.3, 2^16 22.9/25.6, 2^17
+// 37.8/41.6, 2^18 69.4/78.3, 2^19 123/147; 64-word rows 2^15 53.4/52.6, 2^16
+// 73.4/98.4, 2^17 131/164, 2^19 467/604; nodes 2^16 16.5/17.0, 2^17 27.2/27.3,
+// 2^18 45.1/51.0, 2^19 84.4/95.2.  A tensor launch takes an SM's whole register
+// file and thread-per-row launches of these sizes do not, so where several
+// streams share the GPU the lines lie one size above the break-even alone (32
+// jobs of 2^14..2^20 evaluations on 8 streams: 8.95 ms, 9.1 ms with the lines
+// one size lower).
 static bool leaves_on_tensor(size_t n_rows, int row_len) {
   return n_rows >= (row_len <= 16 ? (size_t)1 << 17 : (size_t)1 << 16);
 }

@@ -41,13 +41,13 @@ __device__ __forceinline__ void load_chunk(const uint32_t *__restrict__ row, int
 }
 
 template <bool VEC>
-__global__ void __launch_bounds__(P2T_THREADS, 1)
+__global__ void __launch_bounds__(p2t_threads<24>, 1)
     hash_rows_tensor_kernel(const uint32_t *__restrict__ rows, size_t n_rows, int row_len,
                             uint32_t *__restrict__ digests, const Tri tri, unsigned int *err) {
   extern __shared__ __align__(128) unsigned char sm[];
   P2Tile<24> t = p2t_begin<24>(sm, g_tab24, err);
   pdl_wait();
-  const size_t tiles = (n_rows + 127) / 128, step = (size_t)gridDim.x * P2T_TILES;
+  const size_t tiles = (n_rows + 127) / 128, step = (size_t)gridDim.x * P2Mat<24>::TILES;
   const int lane_row = threadIdx.x & 127;
   size_t tile = (size_t)(threadIdx.x >> 7) * gridDim.x + blockIdx.x;
   uint32_t x[16];
@@ -120,16 +120,16 @@ __global__ void __launch_bounds__(P2T_THREADS, 1)
     }
     tile += step;
   }
-  p2t_end(sm, P2Mat<24>::bytes);
+  p2t_end<24>(sm);
 }
 
-__global__ void __launch_bounds__(P2T_THREADS, 1)
+__global__ void __launch_bounds__(p2t_threads<16>, 1)
     compress_level_tensor_kernel(const uint32_t *__restrict__ src, uint32_t *__restrict__ dst,
                                  size_t half, const Tri tri, unsigned int *err) {
   extern __shared__ __align__(128) unsigned char sm[];
   P2Tile<16> t = p2t_begin<16>(sm, g_tab16, err);
   pdl_wait();
-  const size_t tiles = (half + 127) / 128, step = (size_t)gridDim.x * P2T_TILES;
+  const size_t tiles = (half + 127) / 128, step = (size_t)gridDim.x * P2Mat<16>::TILES;
   const int lane_row = threadIdx.x & 127;
   size_t tile = (size_t)(threadIdx.x >> 7) * gridDim.x + blockIdx.x;
   uint4 a0, a1, b0, b1;
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(P2T_THREADS, 1)
     }
     tile += step;
   }
-  p2t_end(sm, P2Mat<16>::bytes);
+  p2t_end<16>(sm);
 }
 
 Tri tri_of(int width) {
@@ -205,16 +205,16 @@ void hash_rows_tensor(const uint32_t *rows, size_t n_rows, int row_len, uint32_t
   const bool vec = row_len % 4 == 0 && ((uintptr_t)rows & 15) == 0;
   static const Tri tri = tri_of(24);
   if (vec)
-    launch(hash_rows_tensor_kernel<true>, grid_of(n_rows), P2T_THREADS, p2t_smem<24>(), st, rows,
+    launch(hash_rows_tensor_kernel<true>, grid_of(n_rows), p2t_threads<24>, p2t_smem<24>(), st, rows,
            n_rows, row_len, digests, tri, g_wait_error);
   else
-    launch(hash_rows_tensor_kernel<false>, grid_of(n_rows), P2T_THREADS, p2t_smem<24>(), st, rows,
+    launch(hash_rows_tensor_kernel<false>, grid_of(n_rows), p2t_threads<24>, p2t_smem<24>(), st, rows,
            n_rows, row_len, digests, tri, g_wait_error);
 }
 
 void compress_level_tensor(const uint32_t *src, uint32_t *dst, size_t half, cudaStream_t st) {
   static const Tri tri = tri_of(16);
-  launch(compress_level_tensor_kernel, grid_of(half), P2T_THREADS, p2t_smem<16>(), st, src, dst,
+  launch(compress_level_tensor_kernel, grid_of(half), p2t_threads<16>, p2t_smem<16>(), st, src, dst,
          half, tri, g_wait_error);
 }
 

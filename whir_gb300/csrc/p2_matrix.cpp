@@ -165,7 +165,7 @@ struct Builder {
         form_columns(L::blk_off(q), 16, 4 * i, z[4 * q + i], 4 * q);
     for (int i = 0; i < W; i++) {
       s[i].k = kb::add(s[i].k, pc.ext_rc[4][i]);
-      form_columns(L::fin_off(i / 8), 32, 4 * (i % 8), s[i], L::RP);
+      form_columns(L::fin_off(i / L::FW), 4 * L::FW, 4 * (i % L::FW), s[i], L::RP);
     }
     for (int d = 0; d < 3; d++) {  // z_(d+1)'s weight on internal output 0
       const uint32_t c = z[d + 1].c[W];

@@ -41,7 +41,9 @@ struct P2Mat {
   static constexpr int NL = W == 16 ? 16 : 32;  // columns of one half of a light layer
   static constexpr int NBLK = (RP + 3) / 4;     // blocks of four internal rounds
   static constexpr int NCST = 8;                // light layers (initial, after rounds 0-2, 4-7)
-  static constexpr int NFIN = W / 8;            // final-state chunks of 8 words
+  static constexpr int TILES = W == 16 ? 5 : 4;  // 128-row tiles per CTA
+  static constexpr int FW = W == 16 ? 4 : 8;    // words per final-state chunk
+  static constexpr int NFIN = W / FW;
   static constexpr int YSTEPS = 5;              // steps over internal outputs 0..19
   // tables, in bytes from the start
   KB_HD static constexpr int step_bytes(int n) { return n * 32; }
@@ -53,9 +55,11 @@ struct P2Mat {
   KB_HD static constexpr int blk_off(int q) {
     return blk0_off + (q * (1 + 2 * KX) + q * (q - 1) / 2) * step_bytes(16);
   }
-  KB_HD static constexpr int fin_off(int c) { return blk_off(NBLK) + c * fin_steps * step_bytes(32); }
+  KB_HD static constexpr int fin_off(int c) {
+    return blk_off(NBLK) + c * fin_steps * step_bytes(4 * FW);
+  }
   static constexpr int bytes = fin_off(NFIN);
-  // tensor-memory columns of one 128-row tile (128 in all): the W words' low
+  // tensor-memory columns of one 128-row tile: the W words' low
   // byte pairs, their high ones, the constant slots with the internal
   // outputs 20.. (2 columns a word, constants in the last two), the internal
   // outputs 0..19, the sums.  A light layer's 2 NL sums overlie the internal
@@ -64,8 +68,9 @@ struct P2Mat {
   static constexpr int COL_C = 2 * W;
   static constexpr int COL_Y = COL_C + 8;
   static constexpr int COL_D = COL_Y + 8 * YSTEPS;
-  static constexpr int COL_DX = W == 24 ? 64 : COL_D;
-  static_assert(COL_D + 32 <= 128 && COL_DX + 2 * NL <= 128, "tile columns");
+  static constexpr int COLS = COL_D + 4 * FW;
+  static constexpr int COL_DX = COLS - 2 * NL;
+  static_assert(COL_DX >= COL_Y && TILES * COLS <= 512, "tile columns");
 };
 
 // exponent bits of the sums: 2^23 units of 2^-19 (light layers) or 2^-16

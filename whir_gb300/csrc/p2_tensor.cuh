@@ -15,8 +15,12 @@
 //
 // The operands and sums of a tile live in its 128 tensor-memory columns, lane
 // = row, so a thread reads and writes only its own row and no data crosses
-// threads.  A CTA runs four tiles (512 columns, all of an SM's), which hide
-// one another's waits; the tables (86 KB at width 24) are read once per CTA.
+// threads.  A CTA runs as many tiles as an SM's 512 columns hold, four of 128
+// or (width 16) five of 96, which hide one another's waits: a permutation
+// waits for the matrix unit some 20 times, 350 to 400 cycles each.  (Five
+// tiles against four, 2^18 nodes 49.5 -> 45.1 us, 2^19 87.6 -> 84.4; width 24
+// needs 112 columns at least.)  The tables (86 KB at width 24) are read once
+// per CTA.
 #pragma once
 #include "launch.cuh"
 #include "p2_matrix.h"
@@ -24,8 +28,8 @@
 namespace whir {
 namespace gpu {
 
-constexpr int P2T_TILES = 4;  // 128-row tiles per CTA
-constexpr int P2T_THREADS = 128 * P2T_TILES;
+template <int W>
+constexpr int p2t_threads = 128 * P2Mat<W>::TILES;
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -178,7 +182,7 @@ struct P2Tile {
       parity ^= 1u;
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
-    asm volatile("bar.sync %0, 128;" ::"r"(bar + P2T_TILES) : "memory");
+    asm volatile("bar.sync %0, 128;" ::"r"(bar + L::TILES) : "memory");
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   }
 
@@ -294,26 +298,27 @@ struct P2Tile {
       }
     }
     between();
-    // the state after the internal rounds, 8 words at a time, through round
-    // 4's S-boxes; the next 8 words' sums run meanwhile
+    // the state after the internal rounds, FW words at a time, through round
+    // 4's S-boxes; the next words' sums run meanwhile
     uint32_t u[W / 8][8];
-    start([&] { forms<32>(tab + L::fin_off(0) / 16, L::YSTEPS); });
+    start([&] { forms<4 * L::FW>(tab + L::fin_off(0) / 16, L::YSTEPS); });
 #pragma unroll
     for (int c = 0; c < L::NFIN; c++) {
       finish();
-      uint32_t b0[16], b1[16];
-      tm_ld16(b0, row + L::COL_D);
-      tm_ld16(b1, row + L::COL_D + 16);
-      tm_ld_wait();
-      tm_loaded(b0);
-      tm_loaded(b1);
-      if (c + 1 < L::NFIN) start([&] { forms<32>(tab + L::fin_off(c + 1) / 16, L::YSTEPS); });
+      uint32_t b[L::FW / 4][16];
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
-        const uint32_t(&b)[16] = i < 4 ? b0 : b1;
-        const int k = 4 * (i & 3);
-        u[c][i] =
-            (uint32_t)p2t_sbox(p2t_reduce(p2t_form(b[k], b[k + 1], b[k + 2], b[k + 3]))) + kb::P;
+      for (int g = 0; g < L::FW / 4; g++) tm_ld16(b[g], row + L::COL_D + 16 * g);
+      tm_ld_wait();
+#pragma unroll
+      for (int g = 0; g < L::FW / 4; g++) tm_loaded(b[g]);
+      if (c + 1 < L::NFIN)
+        start([&] { forms<4 * L::FW>(tab + L::fin_off(c + 1) / 16, L::YSTEPS); });
+#pragma unroll
+      for (int i = 0; i < L::FW; i++) {
+        const uint32_t(&d)[16] = b[i / 4];
+        const int k = 4 * (i & 3), w = L::FW * c + i;
+        u[w / 8][w % 8] =
+            (uint32_t)p2t_sbox(p2t_reduce(p2t_form(d[k], d[k + 1], d[k + 2], d[k + 3]))) + kb::P;
       }
     }
 #pragma unroll
@@ -345,7 +350,7 @@ __device__ __forceinline__ uint32_t p2t_unsigned(int32_t v) {
 // the tensor-memory address.
 template <int W>
 constexpr size_t p2t_smem() {
-  return P2Mat<W>::bytes + 8 * P2T_TILES + 16;
+  return P2Mat<W>::bytes + 8 * (P2Mat<W>::TILES + 1) + 16;
 }
 template <int W>
 __device__ __forceinline__ P2Tile<W> p2t_begin(unsigned char *sm, const uint4 *table,
@@ -353,16 +358,16 @@ __device__ __forceinline__ P2Tile<W> p2t_begin(unsigned char *sm, const uint4 *t
   using L = P2Mat<W>;
   static_assert(L::bytes % 16 == 0, "table copy");
   uint64_t *bars = reinterpret_cast<uint64_t *>(sm + L::bytes);
-  uint32_t *addr = reinterpret_cast<uint32_t *>(bars + P2T_TILES);
+  uint32_t *addr = reinterpret_cast<uint32_t *>(bars + L::TILES);
   uint4 *dst = reinterpret_cast<uint4 *>(sm);
-  for (int i = threadIdx.x; i < L::bytes / 16; i += P2T_THREADS) dst[i] = __ldg(table + i);
-  if (threadIdx.x < P2T_TILES)
+  for (int i = threadIdx.x; i < L::bytes / 16; i += p2t_threads<W>) dst[i] = __ldg(table + i);
+  if (threadIdx.x < L::TILES)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bars + threadIdx.x))
                  : "memory");
   if (threadIdx.x < 32) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_addr(addr)),
-                 "r"(128 * P2T_TILES)
+                 "r"(512)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
@@ -376,7 +381,7 @@ __device__ __forceinline__ P2Tile<W> p2t_begin(unsigned char *sm, const uint4 *t
   // warp numbers and addresses as warp-uniform values (see mma_step)
   const int wid = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int tile = wid >> 2, warp = wid & 3;
-  t.tile = __shfl_sync(0xffffffffu, *addr, 0) + 128 * tile;
+  t.tile = __shfl_sync(0xffffffffu, *addr, 0) + L::COLS * tile;
   t.row = t.tile + ((uint32_t)(32 * warp) << 16);
   t.tab = smem_addr(sm) >> 4;
   t.mbar = smem_addr(bars + tile);
@@ -390,15 +395,16 @@ __device__ __forceinline__ P2Tile<W> p2t_begin(unsigned char *sm, const uint4 *t
   tm_st8(t.row + L::COL_C, c);
   return t;
 }
-__device__ __forceinline__ void p2t_end(unsigned char *sm, size_t table_bytes) {
+template <int W>
+__device__ __forceinline__ void p2t_end(unsigned char *sm) {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (threadIdx.x < 32) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t a = *reinterpret_cast<uint32_t *>(sm + table_bytes + 8 * P2T_TILES);
+    const uint32_t a = *reinterpret_cast<uint32_t *>(sm + P2Mat<W>::bytes + 8 * P2Mat<W>::TILES);
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(a),
-                 "r"(128 * P2T_TILES));
+                 "r"(512));
   }
 }
 
