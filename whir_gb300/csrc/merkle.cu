@@ -52,10 +52,10 @@ cudaError_t init_poseidon2_tables() {
 // are 128 rows and 608 of them (760 of nodes) fill the GPU; a tile takes 9.2 us
 // per width-24 permutation alone on its SM and 16.5 us among four, so launches
 // of few tiles per SM gain nothing over one thread per row.  Measured, tensor
-// against thread, us: 16-word rows 2^15 16.9/14.3, 2^16 22.9/25.6, 2^17
-// 37.8/41.6, 2^18 69.4/78.3, 2^19 123/147; 64-word rows 2^15 53.4/52.6, 2^16
-// 73.4/98.4, 2^17 131/164, 2^19 467/604; nodes 2^16 16.5/17.0, 2^17 27.2/27.3,
-// 2^18 45.1/51.0, 2^19 84.4/95.2.  A tensor launch takes an SM's whole register
+// against thread, us: 16-word rows 2^15 16.9/13.8, 2^16 22.3/24.4, 2^17
+// 36.0/39.7, 2^18 66.0/74.9, 2^19 117/141; 64-word rows 2^15 52.1/50.1, 2^16
+// 70.3/93.9, 2^17 124/156, 2^19 446/577; nodes 2^16 15.9/16.3, 2^17 26.9/26.0,
+// 2^18 44.0/48.8, 2^19 82.9/91.0.  A tensor launch takes an SM's whole register
 // file and thread-per-row launches of these sizes do not, so where several
 // streams share the GPU the lines lie one size above the break-even alone (32
 // jobs of 2^14..2^20 evaluations on 8 streams: 8.95 ms, 9.1 ms with the lines

@@ -17,7 +17,7 @@ __device__ uint4 g_tab24[P2Mat<24>::bytes / 16];
 unsigned int *g_wait_error;  // pinned, set by a kernel whose wait ran out
 
 struct Tri {
-  int32_t v[3];
+  int32_t v[4];
 };
 
 // Row r of a tile is one leaf: chunks of 16 words overwrite the rate, each
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(p2t_threads<16>, 1)
 
 Tri tri_of(int width) {
   Tri t;
-  for (int i = 0; i < 3; i++) t.v[i] = p2_tables(width).tri[i];
+  for (int i = 0; i < 4; i++) t.v[i] = p2_tables(width).tri[i];
   return t;
 }
 unsigned grid_of(size_t n) {

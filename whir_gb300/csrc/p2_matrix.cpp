@@ -1,6 +1,7 @@
 // Host construction of the tensor-core Poseidon2 tables (see p2_matrix.h).
 #include "p2_matrix.h"
 
+#include <cmath>
 #include <mutex>
 #include <stdexcept>
 
@@ -161,15 +162,29 @@ struct Builder {
       for (int i = 0; i < W; i++) s[i] = sum + scaled(s[i], pc.diag[i]);
     }
     for (int q = 0; q < L::NBLK; q++)
-      for (int i = 0; i < 4 && 4 * q + i < L::RP; i++)
-        form_columns(L::blk_off(q), 16, 4 * i, z[4 * q + i], 4 * q);
+      for (int i = 0; i < L::BLK && L::BLK * q + i < L::RP; i++)
+        form_columns(L::blk_off(q), L::NB, 4 * i, z[L::BLK * q + i], L::BLK * q);
     for (int i = 0; i < W; i++) {
       s[i].k = kb::add(s[i].k, pc.ext_rc[4][i]);
       form_columns(L::fin_off(i / L::FW), 4 * L::FW, 4 * (i % L::FW), s[i], L::RP);
     }
-    for (int d = 0; d < 3; d++) {  // z_(d+1)'s weight on internal output 0
-      const uint32_t c = z[d + 1].c[W];
+    if (z[1].c[W] != kb::neg(kb::ONE)) throw std::logic_error("p2 tables: next round's weight");
+    for (int d = 0; d + 2 < L::BLK; d++) {  // z_(d+2)'s weight on internal output 0
+      const uint32_t c = z[d + 2].c[W];
       t.tri[d] = c > kb::P / 2 ? (int32_t)(c - kb::P) : (int32_t)c;
+    }
+    // The block's values stay in range (units of 2^31; a signed reduction of v
+    // ends within |v| / 2^32 + p / 2).  Round i's form with the outputs up to
+    // two rounds before ends within (-p, p); less the output before, both
+    // canonical, the S-box's operand does too.
+    const double p = kb::P / 2147483648.;
+    double y[8];
+    for (int i = 0; i < L::BLK; i++) {
+      double v = 1e-4;  // the form itself, below 2^49
+      for (int j = 0; j + 1 < i; j++) v += std::abs(t.tri[i - 2 - j] / 2147483648.) * y[j];
+      const double f = v / 2 + p / 2, x = i ? p : f, r = x * x / 2 + p / 2;
+      if (f > p || r > p) throw std::logic_error("p2 tables: block range");
+      y[i] = r * x / 2 + p / 2;
     }
   }
 

@@ -39,7 +39,9 @@ struct P2Mat {
   static constexpr int RP = W == 16 ? 20 : 23;
   static constexpr int KX = W / 8;              // steps over the low (or high) byte pairs
   static constexpr int NL = W == 16 ? 16 : 32;  // columns of one half of a light layer
-  static constexpr int NBLK = (RP + 3) / 4;     // blocks of four internal rounds
+  static constexpr int BLK = W == 16 ? 4 : 6;   // internal rounds per block
+  static constexpr int NBLK = (RP + BLK - 1) / BLK;
+  static constexpr int NB = W == 16 ? 16 : 32;  // columns of a block's forms, 4 each
   static constexpr int NCST = 8;                // light layers (initial, after rounds 0-2, 4-7)
   static constexpr int TILES = W == 16 ? 5 : 4;  // 128-row tiles per CTA
   static constexpr int FW = W == 16 ? 4 : 8;    // words per final-state chunk
@@ -47,13 +49,16 @@ struct P2Mat {
   static constexpr int YSTEPS = 5;              // steps over internal outputs 0..19
   // tables, in bytes from the start
   KB_HD static constexpr int step_bytes(int n) { return n * 32; }
-  KB_HD static constexpr int blk_steps(int q) { return 1 + 2 * KX + q; }
+  // steps over the outputs of the blocks before block q
+  KB_HD static constexpr int blk_ysteps(int q) { return (BLK * q + 3) / 4; }
   static constexpr int fin_steps = 1 + 2 * KX + YSTEPS;
   static constexpr int ext_off = 0;
   static constexpr int cst_off = KX * step_bytes(NL);
   static constexpr int blk0_off = cst_off + NCST * step_bytes(2 * NL);
   KB_HD static constexpr int blk_off(int q) {
-    return blk0_off + (q * (1 + 2 * KX) + q * (q - 1) / 2) * step_bytes(16);
+    int off = blk0_off;
+    for (int i = 0; i < q; i++) off += (1 + 2 * KX + blk_ysteps(i)) * step_bytes(NB);
+    return off;
   }
   KB_HD static constexpr int fin_off(int c) {
     return blk_off(NBLK) + c * fin_steps * step_bytes(4 * FW);
@@ -68,7 +73,7 @@ struct P2Mat {
   static constexpr int COL_C = 2 * W;
   static constexpr int COL_Y = COL_C + 8;
   static constexpr int COL_D = COL_Y + 8 * YSTEPS;
-  static constexpr int COLS = COL_D + 4 * FW;
+  static constexpr int COLS = COL_D + (4 * FW > NB ? 4 * FW : NB);
   static constexpr int COL_DX = COLS - 2 * NL;
   static_assert(COL_DX >= COL_Y && TILES * COLS <= 512, "tile columns");
 };
@@ -82,9 +87,9 @@ constexpr uint32_t P2M_CONST1 = 0x00000100u;
 
 struct P2Tables {
   std::vector<uint16_t> halves;  // P2Mat<W>::bytes / 2
-  // Montgomery words, centred: weight of an internal output on word 0 one,
-  // two and three rounds later (within a block)
-  int32_t tri[3];
+  // Montgomery words, centred: weight of an internal output on word 0 two,
+  // three, .. rounds later (within a block); one round later it is -1
+  int32_t tri[4];
 };
 // Built once per width from the permutation's constants; throws if a sum
 // could leave its exact range.

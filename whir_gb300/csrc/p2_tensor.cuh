@@ -6,10 +6,10 @@
 // instructions of a width-24 permutation some 2 400 are S-box products, the
 // rest adds, shifts and their corrections.  Here a light layer is one small
 // integer matrix product, and the 20 or 23 internal rounds become blocks of
-// four: word 0 before each round is a linear form of earlier S-box outputs,
-// one matrix product per block gives four of them up to the block's own
-// outputs, and one more gives the state after the last round (p2_matrix.h has
-// the tables and the proof that every sum is exact).  A thread splits a word
+// four or (width 24) six: word 0 before each round is a linear form of earlier
+// S-box outputs, one matrix product per block gives all of them up to the
+// block's own outputs, and one more gives the state after the last round
+// (p2_matrix.h has the tables and the proof that every sum is exact).  A thread splits a word
 // into operands with two byte permutes, and takes a light layer's word from
 // its two sums with three instructions and a form's from its four with six.
 //
@@ -108,6 +108,31 @@ __device__ __forceinline__ int32_t p2t_reduce(int64_t v) {
 __device__ __forceinline__ int32_t p2t_sbox(int32_t x) {
   const int32_t r = p2t_reduce((int64_t)x * x);
   return p2t_reduce((int64_t)r * x);
+}
+// N of them side by side, plus p: step by step through all, which the volatile
+// statements hold the compiler to (one after the other, 2^19 rows of 64 words
+// 465 us; in twos 455, fours 451, eights 449)
+template <int N>
+__device__ __forceinline__ void p2t_sboxes(int32_t (&x)[N]) {
+  int64_t p[N];
+  int32_t t[N];
+#pragma unroll
+  for (int i = 0; i < N; i++) asm volatile("mul.wide.s32 %0, %1, %1;" : "=l"(p[i]) : "r"(x[i]));
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+#pragma unroll
+    for (int i = 0; i < N; i++)
+      asm volatile("mul.lo.s32 %0, %1, %2;" : "=r"(t[i]) : "r"((int32_t)p[i]), "r"(kb::MU));
+#pragma unroll
+    for (int i = 0; i < N; i++)
+      asm volatile("mul.hi.s32 %0, %1, %2;" : "=r"(t[i]) : "r"(t[i]), "r"(kb::P));
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      const uint32_t r = (uint32_t)(p[i] >> 32) - (uint32_t)t[i];
+      if (h) x[i] = (int32_t)(r + kb::P);
+      else asm volatile("mul.wide.s32 %0, %1, %2;" : "=l"(p[i]) : "r"(x[i]), "r"(r));
+    }
+  }
 }
 // a light layer's word from the bits of its two sums (p2_matrix.cpp chooses
 // the constants so that the result is the word in a signed register)
@@ -245,13 +270,38 @@ struct P2Tile {
     tm_ld_wait();
 #pragma unroll
     for (int g = 0; g < W / 8; g++) {
+      int32_t x[8];
       uint32_t u[8];
       tm_loaded(a[g]);
       tm_loaded(b[g]);
 #pragma unroll
-      for (int i = 0; i < 8; i++)
-        u[i] = (uint32_t)p2t_sbox(p2t_light_word(a[g][i], b[g][i])) + kb::P;
+      for (int i = 0; i < 8; i++) x[i] = p2t_light_word(a[g][i], b[g][i]);
+      p2t_sboxes(x);
+#pragma unroll
+      for (int i = 0; i < 8; i++) u[i] = (uint32_t)x[i];
       put_words(8 * g, u);
+    }
+  }
+
+  // Block q's outputs (two columns each; zeros behind them) as operands of the
+  // blocks after it, which read whole steps of four: the columns there hold a
+  // light layer's sums until an output is put.  Outputs 20.. share the
+  // constants' step.
+  __device__ __forceinline__ void put_outputs(int q, const uint32_t (&o)[16]) const {
+    const uint32_t at = row + L::COL_Y + 2 * L::BLK * q;
+    const uint32_t o0[8] = {o[0], o[1], o[2], o[3], o[4], o[5], o[6], o[7]};
+    if constexpr (L::BLK == 4) {
+      if (q < L::YSTEPS) tm_st8(at, o0);
+    } else if (q < 3) {
+      const uint32_t o1[8] = {o[8], o[9], o[10], o[11], 0, 0, 0, 0};
+      tm_st8(at, o0);
+      tm_st8(at + 8, o1);
+    } else {
+      tm_st2(at, o[0], o[1]);
+      tm_st2(at + 2, o[2], o[3]);
+      tm_st2(row + L::COL_C, o[4], o[5]);
+      tm_st2(row + L::COL_C + 2, o[6], o[7]);
+      tm_st2(row + L::COL_C + 4, o[8], o[9]);
     }
   }
 
@@ -259,7 +309,7 @@ struct P2Tile {
   // the result (signed, |v| < 2^31, congruent).  `between` runs once the
   // state needs few registers (input of the next permutation is fetched there).
   template <class F>
-  __device__ __forceinline__ void permute(const int32_t (&tri)[3], F &&between) {
+  __device__ __forceinline__ void permute(const int32_t (&tri)[4], F &&between) {
     start([&] { light(0); });
     finish();
 #pragma unroll 1
@@ -271,31 +321,32 @@ struct P2Tile {
     sbox_words();
 #pragma unroll 1
     for (int q = 0; q < L::NBLK; q++) {
-      start([&] { forms<16>(tab + L::blk_off(q) / 16, q); });
+      start([&] { forms<L::NB>(tab + L::blk_off(q) / 16, L::blk_ysteps(q)); });
       finish();
-      uint32_t b[16];
+      uint32_t b[16], b2[8] = {};
       tm_ld16(b, row + L::COL_D);
+      if constexpr (L::BLK == 6) tm_ld8(b2, row + L::COL_D + 16);
       tm_ld_wait();
       tm_loaded(b);
-      uint32_t o[8];
-      int32_t y[4];
+      if constexpr (L::BLK == 6) tm_loaded(b2);
+      uint32_t o[16] = {};
+      int32_t y[L::BLK];
+      uint32_t yc = 0;  // the last output, canonical
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        int64_t x = p2t_form(b[4 * i], b[4 * i + 1], b[4 * i + 2], b[4 * i + 3]);
+      for (int i = 0; i < L::BLK; i++) {
+        const uint32_t *d = i < 4 ? b + 4 * i : b2 + 4 * (i - 4);
+        int64_t x = p2t_form(d[0], d[1], d[2], d[3]);
 #pragma unroll
-        for (int j = 0; j < i; j++) x += (int64_t)tri[i - 1 - j] * y[j];
-        y[i] = p2t_sbox(p2t_reduce(x));
-        const uint32_t u = (uint32_t)y[i] + kb::P;
-        o[2 * i] = p2t_low(u);
-        o[2 * i + 1] = p2t_high(u);
+        for (int j = 0; j + 1 < i; j++) x += (int64_t)tri[i - 2 - j] * y[j];
+        int32_t z = p2t_reduce(x);
+        // the output before weighs -1 (p2_matrix.cpp), so it needs no product
+        if (i) z = (int32_t)(kb::umin((uint32_t)z, (uint32_t)z + kb::P) - yc);
+        y[i] = p2t_sbox(z);
+        yc = kb::umin((uint32_t)y[i], (uint32_t)y[i] + kb::P);
+        o[2 * i] = p2t_low(yc);
+        o[2 * i + 1] = p2t_high(yc);
       }
-      if (4 * q + 4 <= 4 * L::YSTEPS) {
-        tm_st8(row + L::COL_Y + 8 * q, o);
-      } else {  // outputs 20..22 share the constants' step
-        tm_st2(row + L::COL_C, o[0], o[1]);
-        tm_st2(row + L::COL_C + 2, o[2], o[3]);
-        tm_st2(row + L::COL_C + 4, o[4], o[5]);
-      }
+      put_outputs(q, o);
     }
     between();
     // the state after the internal rounds, FW words at a time, through round
