@@ -517,10 +517,10 @@ struct BatchProver::Impl {
     }
   }
 
-  // w[off ..] += eq(point) * scale for each instance's points (the same
-  // count per instance), one table launch and one addition launch
+  // w[off ..] += eq(point) * scale (write: =) for each instance's points (the
+  // same count per instance), one table launch and one addition launch
   void add_eqs(E4 *w, int kt, const std::vector<std::vector<std::vector<E4>>> &pts,
-               const std::vector<std::vector<E4>> &scales) {
+               const std::vector<std::vector<E4>> &scales, bool write = false) {
     const int nt = (int)pts[0].size();
     if (nt == 0) return;
     const int s = kt / 2;
@@ -541,7 +541,7 @@ struct BatchProver::Impl {
     cuda_check(gpu::eq_tables(stage_devp<E4>(po), stage_devp<E4>(so), B * nt, kt, s, eqbuf.as<E4>(),
                               st()),
                "eq_tables");
-    cuda_check(gpu::add_eq_batch(w, kt, eqbuf.as<E4>(), nt, B, st()), "add_eq");
+    cuda_check(gpu::add_eq_batch(w, kt, eqbuf.as<E4>(), nt, B, st(), write), "add_eq");
   }
 
   // w += sum_t scales_t var_t^i per instance (ragged counts)
@@ -634,8 +634,9 @@ struct BatchProver::Impl {
     cuda_check(gpu::compress_lo_batch(stacked.as<uint32_t>(), k, ks, stage_devp<E4>(ro), B,
                                       (size_t)1 << k, P(), st()),
                "compress_lo");
-    cuda_check(cudaMemsetAsync(W(), 0, Bz * N * sizeof(E4), st()), "memset");
-    add_eqs(W(), kc, pts, scl);
+    // the claims write W; without any it starts as zeros
+    if (pts[0].empty()) cuda_check(cudaMemsetAsync(W(), 0, Bz * N * sizeof(E4), st()), "memset");
+    else add_eqs(W(), kc, pts, scl, true);
   }
 
   // ---- queries (MerkleTree::query, poseidon_packed.rs:145-233) ----

@@ -148,10 +148,12 @@ cudaError_t compress_lo(const uint32_t *poly, int k, const Point &rs, kb::E4 *ou
 // w[i] += sum_t lo_t[i & (2^s-1)] * hi_t[i >> s] for n_tables split eq tables
 // stored back to back (lo0, hi0, lo1, hi1, ...), s = k / 2, each lo 2^s and
 // hi 2^(k-s) entries.
-cudaError_t add_eq(kb::E4 *w, int k, const kb::E4 *tables, int n_tables, cudaStream_t st);
+cudaError_t add_eq(kb::E4 *w, int k, const kb::E4 *tables, int n_tables, cudaStream_t st,
+                   bool write = false);
 // w[i] += sum_t scale_t eq(z_t)[i] for n <= EqArgs::N points of k coordinates,
 // the tables formed by the kernel; add_eq_by_points: the sizes it is for
-cudaError_t add_eq_points(kb::E4 *w, int k, const EqArgs &a, int n, cudaStream_t st);
+cudaError_t add_eq_points(kb::E4 *w, int k, const EqArgs &a, int n, cudaStream_t st,
+                          bool write = false);
 bool add_eq_by_points(int k, int n);
 // w[i] += sum_t scale_t * var_t^i  (pow::combine_pows(_scaled), combine.rs:408-468);
 // tab: add_pows_scratch_words(k, n) words for the split power tables
@@ -236,7 +238,7 @@ cudaError_t compress_lo_batch(const uint32_t *poly, int k, int ks, const kb::E4 
                               size_t poly_stride, kb::E4 *out, cudaStream_t st);
 // instance y: w + y 2^k and n_tables tables from tables + y n_tables (2^s + 2^(k-s))
 cudaError_t add_eq_batch(kb::E4 *w, int k, const kb::E4 *tables, int n_tables, int batch,
-                         cudaStream_t st);
+                         cudaStream_t st, bool write = false);
 // ragged: instance y adds vars[off[y] .. off[y+1]) with their scales into
 // w + y 2^k (off: batch + 1 device ints, max_n the largest count)
 cudaError_t add_pows_batch(kb::E4 *w, int k, const uint32_t *vars, const kb::E4 *scales,

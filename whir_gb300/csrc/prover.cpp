@@ -822,13 +822,15 @@ struct Prover::Impl {
       a.scale[t] = scales[t];
     }
   }
-  // w[off .. off + 2^kt) += eq(point) * scale for several points sharing the range
-  void add_eqs(E4 *w, int kt, const std::vector<std::vector<E4>> &pts, const std::vector<E4> &scales) {
+  // w[off .. off + 2^kt) += eq(point) * scale for several points sharing the
+  // range; write: = instead of +=
+  void add_eqs(E4 *w, int kt, const std::vector<std::vector<E4>> &pts, const std::vector<E4> &scales,
+               bool write = false) {
     if (pts.empty()) return;
     if (gpu::add_eq_by_points(kt, (int)pts.size())) {
       gpu::EqArgs a;
       fill_eq_args(a, pts, scales);
-      cuda_check(gpu::add_eq_points(w, kt, a, (int)pts.size(), st()), "add_eq");
+      cuda_check(gpu::add_eq_points(w, kt, a, (int)pts.size(), st(), write), "add_eq");
       return;
     }
     int s = kt / 2;
@@ -838,7 +840,7 @@ struct Prover::Impl {
     std::vector<const E4 *> pp;
     for (auto &q : pts) pp.push_back(q.data());
     make_eq_tables(pp, kt, scales, s, eqbuf.as<E4>());
-    cuda_check(gpu::add_eq(w, kt, eqbuf.as<E4>(), (int)pts.size(), st()), "add_eq");
+    cuda_check(gpu::add_eq(w, kt, eqbuf.as<E4>(), (int)pts.size(), st(), write), "add_eq");
   }
 
   // w += sum_t scales_t var_t^i; arguments go through the pinned argument
@@ -914,7 +916,6 @@ struct Prover::Impl {
       size_t o = lay[e].index << (pk[id] - ks);
       cuda_check(gpu::compress_lo(poly_dev(id), pk[id], rsp, P() + o, st()), "compress_lo");
     }
-    cuda_check(cudaMemsetAsync(W(), 0, N * sizeof(E4), st()), "memset");
     // group the eq additions by target range
     std::map<std::pair<size_t, int>, std::pair<std::vector<std::vector<E4>>, std::vector<E4>>> groups;
     a = e_one();
@@ -935,7 +936,16 @@ struct Prover::Impl {
       g.second.push_back(scale);
       a = e_mul(a, alpha);
     }
-    for (auto &kv : groups) add_eqs(W() + kv.first.first, kv.first.second, kv.second.first, kv.second.second);
+    // the claims on the whole range write it (without one it starts as zeros),
+    // the others add to their parts
+    auto whole = groups.find({0, kc});
+    if (whole == groups.end())
+      cuda_check(cudaMemsetAsync(W(), 0, N * sizeof(E4), st()), "memset");
+    else
+      add_eqs(W(), kc, whole->second.first, whole->second.second, true);
+    for (auto it = groups.begin(); it != groups.end(); ++it)
+      if (it != whole)
+        add_eqs(W() + it->first.first, it->first.second, it->second.first, it->second.second);
     check_sum("new_prover");
   }
 
@@ -1075,7 +1085,8 @@ struct Prover::Impl {
     cs.omega = two_adic_generator(k_data);
     cs.winv = inv(cs.omega);
     cs.two_inv = inv(from_canonical(2));
-    // device layout in codebuf: G | scales | idx | ws | tw | B | wd | row list
+    // device layout in codebuf: G | ws | tw | B, and what one copy brings:
+    // scales | idx | wd | row list
     size_t g_bytes = 16 * (size_t)n * T, sc_bytes = 16 * (size_t)n, u_bytes = 4 * (((size_t)n + 3) & ~(size_t)3);
     size_t wd_bytes = 4 * ((T + 3) & ~(size_t)3), rl_bytes = 4 * (size_t)n * T;
     size_t need = g_bytes + sc_bytes + 4 * u_bytes + wd_bytes + rl_bytes + 64;
@@ -1085,17 +1096,19 @@ struct Prover::Impl {
     }
     uint8_t *cb = codebuf.as<uint8_t>();
     cs.G = reinterpret_cast<E4 *>(cb);
-    cs.scales = reinterpret_cast<E4 *>(cb + g_bytes);
-    uint32_t *didx = reinterpret_cast<uint32_t *>(cb + g_bytes + sc_bytes);
-    cs.idx = didx;
-    cs.ws = didx + u_bytes / 4;
+    cs.ws = reinterpret_cast<uint32_t *>(cb + g_bytes);
     cs.tw = cs.ws + u_bytes / 4;
     cs.B = cs.tw + u_bytes / 4;
-    uint32_t *dwd = cs.B + u_bytes / 4;
+    cs.scales = reinterpret_cast<E4 *>(cs.B + u_bytes / 4);
+    uint32_t *didx = reinterpret_cast<uint32_t *>(cs.scales + n);
+    cs.idx = didx;
+    uint32_t *dwd = didx + u_bytes / 4;
     cs.wd = dwd;
     uint32_t *drows = dwd + wd_bytes / 4;
-    {
-      std::vector<uint32_t> h((size_t)n * T), hi(n), hw(T);
+    if (n) {
+      std::vector<uint32_t> args((sc_bytes + u_bytes + wd_bytes + rl_bytes) / 4, 0);
+      uint32_t *hi = args.data() + sc_bytes / 4, *hw = hi + u_bytes / 4, *h = hw + wd_bytes / 4;
+      memcpy(args.data(), scales.data(), sc_bytes);
       for (int i = 0; i < n; i++) {
         hi[i] = (uint32_t)idx[i];
         for (size_t t = 0; t < T; t++) h[(size_t)i * T + t] = (uint32_t)((idx[i] & (S - 1)) + t * S);
@@ -1103,10 +1116,7 @@ struct Prover::Impl {
       uint32_t wd = kb::pow(cs.winv, S);
       hw[0] = ONE;
       for (size_t t = 1; t < T; t++) hw[t] = mul(hw[t - 1], wd);
-      upload(drows, h.data(), 4 * h.size());
-      upload(didx, hi.data(), 4 * (size_t)n);
-      upload(dwd, hw.data(), 4 * T);
-      upload(cs.scales, scales.data(), 16 * (size_t)n);
+      upload(cs.scales, args.data(), 4 * args.size());
     }
     gpu::Point rsp;
     rsp.k = (int)rs.size();

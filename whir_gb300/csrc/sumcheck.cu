@@ -16,11 +16,6 @@ namespace gpu {
 
 using kb::E4;
 
-__device__ __forceinline__ void acc_add(unsigned long long *a, const E4 &v) {
-#pragma unroll
-  for (int c = 0; c < 4; c++) atomicAdd(a + c, (unsigned long long)v.c[c]);
-}
-
 // Extension elements through 16-byte accesses when the arrays are 16-byte
 // aligned (VEC; E4 itself only promises 4), word by word otherwise.
 template <bool VEC>
@@ -556,16 +551,17 @@ cudaError_t compress_lo_batch(const uint32_t *poly, int k, int ks, const E4 *rs_
 
 // w[i] += sum_t lo_t[i & mask] * hi_t[i >> s].  Batched: instance y =
 // blockIdx.y adds its n_tables tables (stored after those of instances < y)
-// into w + y n.
+// into w + y n.  write: w[i] = instead of +=, so that a fresh w needs no
+// clearing pass before (2^20 entries: 16 MB written and read less).
 template <bool VEC>
 __global__ void add_eq_kernel(E4 *w, size_t n, int s, size_t n_lo, size_t n_hi,
-                              const E4 *__restrict__ tables, int n_tables) {
+                              const E4 *__restrict__ tables, int n_tables, bool write) {
   pdl_wait();
   w += blockIdx.y * n;
   tables += blockIdx.y * (size_t)n_tables * (n_lo + n_hi);
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (size_t)gridDim.x * blockDim.x) {
-    E4 acc = ld_e4<VEC>(w + i);
+    E4 acc = write ? kb::e_zero() : ld_e4<VEC>(w + i);
     for (int t = 0; t < n_tables; t++) {
       const E4 *lo = tables + t * (n_lo + n_hi), *hi = lo + n_lo;
       acc = kb::e_add(acc, kb::e_mul(ld_e4<VEC>(lo + (i & (n_lo - 1))), ld_e4<VEC>(hi + (i >> s))));
@@ -575,7 +571,7 @@ __global__ void add_eq_kernel(E4 *w, size_t n, int s, size_t n_lo, size_t n_hi,
 }
 
 cudaError_t add_eq_batch(E4 *w, int k, const E4 *tables, int n_tables, int batch,
-                         cudaStream_t st) {
+                         cudaStream_t st, bool write) {
   if (n_tables == 0) return cudaSuccess;
   if (batch < 1 || batch > 65535) return cudaErrorInvalidValue;
   int s = k / 2;
@@ -585,16 +581,16 @@ cudaError_t add_eq_batch(E4 *w, int k, const E4 *tables, int n_tables, int batch
   dim3 grid((unsigned)(g < cap ? g : cap), (unsigned)batch);
   if (aligned16(w) && aligned16(tables))
     launch(add_eq_kernel<true>, grid, T, 0, st, w, n, s, (size_t)1 << s, (size_t)1 << (k - s),
-           tables, n_tables);
+           tables, n_tables, write);
   else
     launch(add_eq_kernel<false>, grid, T, 0, st, w, n, s, (size_t)1 << s, (size_t)1 << (k - s),
-           tables, n_tables);
+           tables, n_tables, write);
   count_launches(1);
   return cudaGetLastError();
 }
 
-cudaError_t add_eq(E4 *w, int k, const E4 *tables, int n_tables, cudaStream_t st) {
-  return add_eq_batch(w, k, tables, n_tables, 1, st);
+cudaError_t add_eq(E4 *w, int k, const E4 *tables, int n_tables, cudaStream_t st, bool write) {
+  return add_eq_batch(w, k, tables, n_tables, 1, st, write);
 }
 
 // w[i] += sum_t scale_t eq(z_t)[i] for at most EqArgs::N points, the tables
@@ -608,7 +604,7 @@ cudaError_t add_eq(E4 *w, int k, const E4 *tables, int n_tables, cudaStream_t st
 template <bool VEC>
 __global__ void __launch_bounds__(256) add_eq_points_kernel(E4 *__restrict__ w, int k,
                                                             const __grid_constant__ EqArgs a,
-                                                            int n) {
+                                                            int n, bool write) {
   pdl_wait();
   __shared__ E4 A[EqArgs::N][16], B[EqArgs::N][16];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -632,7 +628,7 @@ __global__ void __launch_bounds__(256) add_eq_points_kernel(E4 *__restrict__ w, 
   __syncthreads();
   const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
   if (i >> k) return;
-  E4 x = ld_e4<VEC>(w + i);
+  E4 x = write ? kb::e_zero() : ld_e4<VEC>(w + i);
   for (int t = 0; t < n; t++)
     x = kb::e_add(x, kb::e_mul(A[t][threadIdx.x & ((1 << na) - 1)], B[t][threadIdx.x >> na]));
   st_e4<VEC>(w + i, x);
@@ -641,12 +637,12 @@ __global__ void __launch_bounds__(256) add_eq_points_kernel(E4 *__restrict__ w, 
 bool add_eq_by_points(int k, int n) {
   return n <= EqArgs::N && k <= 18 && ((size_t)n << k) <= ((size_t)1 << 18);
 }
-cudaError_t add_eq_points(E4 *w, int k, const EqArgs &a, int n, cudaStream_t st) {
+cudaError_t add_eq_points(E4 *w, int k, const EqArgs &a, int n, cudaStream_t st, bool write) {
   if (n == 0) return cudaSuccess;
   if (n > EqArgs::N || k < 0 || k > EqArgs::K || k > 31) return cudaErrorInvalidValue;
   const unsigned g = k <= 8 ? 1u : 1u << (k - 8);
-  if (aligned16(w)) launch(add_eq_points_kernel<true>, g, 256, 0, st, w, k, a, n);
-  else launch(add_eq_points_kernel<false>, g, 256, 0, st, w, k, a, n);
+  if (aligned16(w)) launch(add_eq_points_kernel<true>, g, 256, 0, st, w, k, a, n, write);
+  else launch(add_eq_points_kernel<false>, g, 256, 0, st, w, k, a, n, write);
   count_launches(1);
   return cudaGetLastError();
 }
