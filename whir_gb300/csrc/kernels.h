@@ -77,14 +77,15 @@ cudaError_t build_tree(uint32_t *nodes, int log_h, cudaStream_t st, uint32_t *ho
 // per query: the leaf row then log_h sibling digests bottom-up
 cudaError_t gather_openings(const uint32_t *rows, int row_len, const uint32_t *nodes, int log_h,
                             const uint32_t *idx, int n, uint32_t *out, cudaStream_t st);
-// the same with at most IdxArgs::N indexes passed by value
+// the same with at most IdxArgs::N indexes passed by value; a pub with a flag
+// raises it when every opening is written (no words)
 struct IdxArgs {
   static constexpr int N = 2048;
   uint32_t idx[N];
 };
 cudaError_t gather_openings_val(const uint32_t *rows, int row_len, const uint32_t *nodes,
                                 int log_h, const IdxArgs &a, int n, uint32_t *out,
-                                cudaStream_t st);
+                                cudaStream_t st, const Publish &pub = Publish());
 // Merkle path checks of many openings (MerkleTree::verify,
 // crates/merkle/src/poseidon_packed.rs:235-257, path check poseidon.rs:22-41):
 // path i's words start at words[d[i].off]: the row (row_len words, hashed as

@@ -694,20 +694,26 @@ __global__ void gather_openings_kernel(const uint32_t *__restrict__ rows, int ro
 // the same with the indexes passed by value
 __global__ void gather_openings_val_kernel(const uint32_t *__restrict__ rows, int row_len,
                                            const uint32_t *__restrict__ nodes, int log_h,
-                                           const __grid_constant__ IdxArgs a, int n,
-                                           uint32_t *__restrict__ out) {
+                                           const __grid_constant__ IdxArgs a,
+                                           uint32_t *__restrict__ out, Publish pub) {
   pdl_wait();
-  int q = blockIdx.x;
-  if (q >= n) return;
-  gather_one(rows, row_len, nodes, log_h, a.idx[q], q, out);
+  gather_one(rows, row_len, nodes, log_h, a.idx[blockIdx.x], (int)blockIdx.x, out);
+  if (!pub.flag) return;
+  __threadfence_system();  // the openings reach host memory before the flag
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(pub.counter, 1u) == gridDim.x - 1) {
+    atomicExch(pub.counter, 0u);
+    __threadfence_system();
+    *reinterpret_cast<volatile unsigned int *>(pub.flag) = pub.seq;
+  }
 }
 
 cudaError_t gather_openings_val(const uint32_t *rows, int row_len, const uint32_t *nodes,
                                 int log_h, const IdxArgs &a, int n, uint32_t *out,
-                                cudaStream_t st) {
+                                cudaStream_t st, const Publish &pub) {
   if (n == 0) return cudaSuccess;
   if (n > IdxArgs::N) return cudaErrorInvalidValue;
-  launch(gather_openings_val_kernel, n, 128, 0, st, rows, row_len, nodes, log_h, a, n, out);
+  launch(gather_openings_val_kernel, n, 128, 0, st, rows, row_len, nodes, log_h, a, out, pub);
   count_launches(1);
   return cudaGetLastError();
 }

@@ -668,6 +668,7 @@ struct Prover::Impl {
     args_pin.reserve((size_t)1 << 20);
     ptsbuf.reserve(64 << 10);
     defer_pin.reserve((size_t)16 << 20);
+    if (acc.bytes() < w.acc) acc_zero = false;
     acc.reserve(w.acc);
     small.reserve(w.small);
     gather.reserve(w.gather);
@@ -695,6 +696,7 @@ struct Prover::Impl {
     svo_finish(c, ks, h);
   }
 
+  bool acc_zero = false;  // the accumulators are all zero (the last proof ended)
   const uint32_t *poly_dev(int id) const { return stacked.as<uint32_t>() + poly_off[id]; }
 
   // claims in layout order: (claim index, layout entry)
@@ -954,7 +956,10 @@ struct Prover::Impl {
   // starts their gather; the rows land in the deferred pinned area (word
   // offset returned, `per` words per index) and are readable after the next
   // sync; the hint bytes are filled in at the end of the proof.
-  size_t query_async(Transcript &ts, const DeviceTree &t, const std::vector<size_t> &idx) {
+  // flagged: the proof's last gather, set when it will raise the published flag
+  // (otherwise the caller syncs)
+  size_t query_async(Transcript &ts, const DeviceTree &t, const std::vector<size_t> &idx,
+                     bool *flagged = nullptr) {
     int n = (int)idx.size();
     if (n == 0) return 0;
     size_t per = (size_t)t.row_len + 8 * (size_t)t.log_h;
@@ -964,8 +969,10 @@ struct Prover::Impl {
       static thread_local gpu::IdxArgs a;
       for (int i = 0; i < n; i++) a.idx[i] = (uint32_t)idx[i];
       cuda_check(gpu::gather_openings_val(t.rows, t.row_len, t.nodes, t.log_h, a, n,
-                                          defer_ptr(off), st()),
+                                          defer_ptr(off), st(),
+                                          flagged ? publish(0) : gpu::Publish()),
                  "gather");
+      if (flagged) *flagged = true;
     } else {
       size_t need = 4 * (size_t)n + 16;
       if (need > gather.bytes()) {
@@ -1204,11 +1211,22 @@ struct Prover::Impl {
       cur_tree = slot;
     }
     Span final_span("final");  // whir.rs:314
-    flush();
-    size_t nf = (size_t)1 << kc;
-    E4 *hf = (E4 *)ctx->pinned(16 * nf);
-    cuda_check(copy_async(*ctx, hf, P(), 16 * nf, cudaMemcpyDeviceToHost), "d2h");
-    sync();
+    const size_t nf = (size_t)1 << kc;
+    E4 *hf = reinterpret_cast<E4 *>((uint8_t *)ctx->pinned(8 * PUB_WORDS + 16 * nf) + 8 * PUB_WORDS);
+    if (pending && nf <= 512) {
+      // one CTA folds straight into pinned memory and raises the flag: no copy
+      // and no stream sync (with the last gather's flag 3 to 15 us of a proof)
+      cuda_check(gpu::sumcheck_round(P(), W(), 2 * nf, true, pending_r, hf, sw[1 - ping].as<E4>(),
+                                     true, acc.as<unsigned long long>(), st(), publish(12)),
+                 "final fold");
+      pending = false;
+      ctx->count_copy(16 * nf, cudaMemcpyDeviceToHost);
+      wait_published();
+    } else {
+      flush();
+      cuda_check(copy_async(*ctx, hf, P(), 16 * nf, cudaMemcpyDeviceToHost), "d2h");
+      sync();
+    }
     std::vector<E4> fp(hf, hf + nf);
     for (auto &e : fp) ts.write_ext(e);
     int kfd, this_rate, prev_rate;
@@ -1216,11 +1234,14 @@ struct Prover::Impl {
     int n_s = n_stir_queries(p.soundness, p.security_level, prev_rate);
     std::vector<size_t> idx = stir_indexes(ts, kfd, n_s);
     const DeviceTree &last = cur_tree >= 0 ? tr[cur_tree] : t0;
-    size_t rows_off = query_async(ts, last, idx);
-    sync();
+    bool flagged = false;
+    size_t rows_off = query_async(ts, last, idx, &flagged);
+    if (flagged) wait_published();
+    else sync();
     check_stir(idx, kfd, rows_off, (size_t)last.row_len + 8 * (size_t)last.log_h, last.row_len,
                cur_tree < 0, cur_tree >= 0 ? round_point : rs, &fp);
     fill_pending_hints(ts);
+    acc_zero = true;
     if (kc != final_rounds) throw WhirError(-1, "final sumcheck size mismatch");
   }
 
@@ -1310,9 +1331,11 @@ void Prover::commit(Transcript &ts, const uint32_t *polys, bool on_device,
   m.pk = poly_k;
   m.make_layout();
   m.reserve();
-  // reductions publish and re-zero their accumulators (Impl::publish); start
-  // every proof from zero
-  cuda_check(cudaMemsetAsync(m.acc.as<void>(), 0, m.acc.bytes(), ctx_->stream()), "memset");
+  // reductions publish and re-zero their accumulators (Impl::publish), so a
+  // finished proof leaves them zero; anything else starts from a memset
+  if (!m.acc_zero)
+    cuda_check(cudaMemsetAsync(m.acc.as<void>(), 0, m.acc.bytes(), ctx_->stream()), "memset");
+  m.acc_zero = false;
   m.claims.clear();
   m.virt.clear();
   cudaStream_t st = ctx_->stream();
