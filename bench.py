@@ -43,17 +43,17 @@ WORKLOAD = dict(k=24, folding=4, rate=2, initial_reduction=1, soundness="Johnson
 METRIC = "proofs/sec and p50/p99 latency, batched/served vs plain, 1 GB300, bit-exact"
 UNIT = "proofs/s"
 # Per-launch DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of the
-# kernel classes, from one ncu capture of a full k = 24 proof (the five
-# leaf-hash launches: 1473.0 MB per proof / 5 launches); the capture, its
-# command and the per-launch figures are kept with the ncu summaries (profiles/).
-NCU_TRAFFIC_BYTES = {"leaf_hash": 294.6e6}
+# leaf-hash launches of a k = 24 proof: 0.975 of the algorithmic bytes (307.0 MB
+# per launch), as ncu counted for 2^20 rows of 64 words (268.6 MB read, 26.0 MB
+# written of 302.0 MB; the capture and its command are in profiles/).
+NCU_TRAFFIC_BYTES = {"leaf_hash": 299.4e6}
 NCU_TRAFFIC_K = 24
 # Thread instructions per width-24 permutation of the leaf hash
-# (smsp__inst_executed.sum * 32 / permutations of hash_rows_fixed<16> on a
-# k = 22 proof, the ncu summary of the leaf hash in profiles/).  With one warp
+# (smsp__inst_executed.sum * 32 / permutations of hash_rows_tensor_kernel on
+# 2^20 rows of 64 words, the same ncu summary in profiles/).  With one warp
 # instruction issued per cycle on each of the 4 sub-partitions of each SM,
 # the issue-bound rate is SMs * 4 * 32 * clock / this.
-LEAF_INSTR_PER_PERM24 = 8087
+LEAF_INSTR_PER_PERM24 = 3940
 GB300_SMS = 152
 
 
@@ -176,8 +176,9 @@ def integer_roofline(k, prof, clk):
             "peak_source": f"{instr} instructions per permutation (the fewer of the structural "
                            f"count and the kernel's, ncu) at {mhz:.0f} MHz, 152 SMs x 4 issue "
                            f"slots of 32 lanes",
-            "note": "the kernel issues fewer instructions than the structural count; the gap "
-                    "to the issue rate is pipe contention (FMA-heavy 87%, ALU 67%, profiles/)"}
+            "note": "the linear layers run on the tensor cores, so the kernel issues far fewer "
+                    "instructions than the structural count; the gap to the issue rate is the "
+                    "FMA-heavy pipe (75%) and the waits for the matrix unit (profiles/)"}
 
 
 def workload_config(k):
