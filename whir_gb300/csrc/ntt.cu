@@ -8,8 +8,8 @@
 // there, three radix-2 stages per step in registers.  When the nonzero input
 // has at most 2^12 rows (every WHIR round after the first, whose rate grows),
 // the codeword is a set of independent coset transforms of that input and
-// also takes one pass.  Otherwise sizes
-// use the four-step split M = M1 * M2:
+// also takes one pass (2^12 of them only when that makes enough tiles).
+// Otherwise sizes use the four-step split M = M1 * M2:
 //   pass 1: for each n2, a size-M1 DFT of x[M2 n1 + n2] (stride M2 rows),
 //           times w_M^(n2 k1), stored at row M2 k1 + n2;
 //   pass 2: for each k1, a size-M2 DFT of the contiguous rows M2 k1 + n2,
@@ -717,7 +717,13 @@ static cudaError_t tile_any(const uint32_t *in, uint32_t *out, int S, size_t wid
                             size_t rows_valid, size_t n_outer, size_t a_in, size_t b_in,
                             size_t a_out, size_t b_out, int pre_log, int tw_log, cudaStream_t st) {
   const bool aligned = (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
-  if (aligned && width % 8 == 0)
+  // Slices of 8 columns read whole 32-byte sectors, but where they leave half
+  // of the SMs idle twice as many of 4 finish sooner (us, 16 columns: 2^11 rows
+  // 9.2 -> 6.8, 2^12 from 2^11 12.7 -> 8.6, 2^10 5.3 -> 4.8).
+  int lg = 0;
+  while (S + lg < 10 && ((size_t)2 << lg) <= n_outer) lg++;
+  const bool few = (width / 8) * (n_outer >> lg) <= 76;
+  if (aligned && width % 8 == 0 && !few)
     return launch_tile_v<8>(in, out, S, width, rows_valid, n_outer, a_in, b_in, a_out, b_out,
                             pre_log, tw_log, st);
   if (aligned && width % 4 == 0)
@@ -741,10 +747,16 @@ static int ceil_log2(size_t x) {
   while (((size_t)1 << l) < x) l++;
   return l;
 }
+// 2^12-row tiles follow each other's steps for 15 us however few they are; up
+// to 64 of them two passes of smaller tiles are faster (us, one pass and two:
+// 2^14 rows of 16 words 15.1 / 11.0, of 64 15.6 / 11.6, 2^15 of 64 15.8 / 16.3).
+static bool coset12_one_pass(int log_h, size_t width) {
+  return width % 4 == 0 && ((width / 4) << (log_h - 12)) > 64;
+}
 bool dft_coset_one_pass(int log_h, size_t h_in, size_t width) {
   if (log_h <= 11) return false;
   const int L0 = ceil_log2(h_in);
-  return log_h - L0 <= 15 && (L0 <= 11 || (L0 == 12 && width % 4 == 0));
+  return log_h - L0 <= 15 && (L0 <= 11 || (L0 == 12 && coset12_one_pass(log_h, width)));
 }
 
 // per-size overrides of the two-pass split (0: default), by log_h and width class
@@ -783,7 +795,7 @@ cudaError_t dft_batch(const uint32_t *in, size_t h_in, size_t width, int log_h, 
     size_t M1 = h >> L0;
     return tile_any(in, out, L0, width, h_in, M1, 0, 1, 1, M1, log_h, 0, st);
   }
-  if (L0 == 12 && log_h - L0 <= 15 && width % 4 == 0 &&
+  if (L0 == 12 && log_h - L0 <= 15 && coset12_one_pass(log_h, width) &&
       (((uintptr_t)in | (uintptr_t)out) & 15) == 0) {
     // the same coset form on 2^12-row tiles of 4 columns (64 KB of shared
     // memory, three CTAs per SM; 8 columns would leave one)
