@@ -157,6 +157,11 @@ WHIR_API int whir_fold_code_rounds(whir_ctx *ctx, const uint32_t *codeword, int 
  * whir.rs:361-522) instead of after reading the whole proof (the order
  * whir_verify_batch uses); the results are the same either way. */
 WHIR_API int whir_debug_set(unsigned flags);
+/* The tensor-core hash kernels bound their waits for the matrix unit (one
+ * second); a kernel whose wait runs out ends in an orderly way, and the call
+ * that launched it returns WHIR_ERR_CUDA.  on != 0: on this context every such
+ * wait counts as run out, to test that path; 0 (the default): none does. */
+WHIR_API int whir_debug_expire_waits(whir_ctx *ctx, int on);
 
 /* Poseidon2KoalaBear<width>::permute_mut on the host (width 16 or 24), with
  * the constants of new_from_rng_128(&mut rng(1000)) used by the harness

@@ -148,6 +148,7 @@ _SIGS = {
                                              ctypes.POINTER(ctypes.c_size_t), ctypes.c_int, u32p,
                                              u32p, u32p, u32p]),
     "whir_debug_set": (ctypes.c_int, [ctypes.c_uint]),
+    "whir_debug_expire_waits": (ctypes.c_int, [vp, ctypes.c_int]),
     "whir_counters": (ctypes.c_int, [vp, ctypes.POINTER(ctypes.c_uint64),
                                      ctypes.POINTER(ctypes.c_uint64),
                                      ctypes.POINTER(ctypes.c_uint64)]),
@@ -528,6 +529,12 @@ def debug_set(flags):
     DEBUG_NVTX (NVTX ranges) and/or DEBUG_VERIFY_INLINE (verify hashes each
     opening where it reads it); 0 turns the debug mode off."""
     _check(lib().whir_debug_set(flags))
+
+
+def debug_expire_waits(ctx, on=True):
+    """whir_debug_expire_waits: let the tensor-core hash kernels of this context
+    give up their waits, to test what follows."""
+    _check(lib().whir_debug_expire_waits(ctx.h, 1 if on else 0))
 
 
 def batch_max(params):

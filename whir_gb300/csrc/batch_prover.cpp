@@ -382,10 +382,11 @@ struct BatchProver::Impl {
                "dft_batch");
     ctx->prof_end(Context::K_DFT, 4.0 * (double)(Bz * (h_in * w + rows * w)));
     ctx->prof_begin(Context::K_LEAF);
-    cuda_check(gpu::hash_rows(codeword, rows * Bz, (int)w, nodes, st()), "hash_rows");
+    cuda_check(gpu::hash_rows(codeword, rows * Bz, (int)w, nodes, st(), ctx->wait_report()),
+               "hash_rows");
     ctx->prof_end(Context::K_LEAF, 4.0 * (double)(Bz * (rows * w + rows * 8)));
     ctx->prof_begin(Context::K_TREE);
-    cuda_check(gpu::build_tree_batch(nodes, log_h, B, st()), "build_tree");
+    cuda_check(gpu::build_tree_batch(nodes, log_h, B, st(), ctx->wait_report()), "build_tree");
     ctx->prof_end(Context::K_TREE, 32.0 * (double)(Bz * (2 * rows - 2 + rows - 1)));
     cuda_check(copy_async(*ctx, roots_pin.data(), nodes + Bz * gpu::level_offset_words(log_h, log_h),
                           32 * Bz, cudaMemcpyDeviceToHost),

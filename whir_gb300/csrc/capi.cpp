@@ -196,9 +196,12 @@ int whir_merkle_commit(whir_ctx *ctx, const uint32_t *rows, int log_h, size_t ro
     t->nodes->reserve(4 * whir::gpu::tree_words(log_h));
     cudaStream_t st = ctx->ctx.stream();
     size_t n = (size_t)1 << log_h;
-    whir::cuda_check(whir::gpu::hash_rows(rows, n, (int)row_len, t->nodes->as<uint32_t>(), st),
+    whir::cuda_check(whir::gpu::hash_rows(rows, n, (int)row_len, t->nodes->as<uint32_t>(), st,
+                                          ctx->ctx.wait_report()),
                      "hash_rows");
-    whir::cuda_check(whir::gpu::build_tree(t->nodes->as<uint32_t>(), log_h, st), "build_tree");
+    whir::cuda_check(whir::gpu::build_tree(t->nodes->as<uint32_t>(), log_h, st,
+                                           ctx->ctx.wait_report()),
+                     "build_tree");
     uint32_t h[8];
     whir::cuda_check(cudaMemcpyAsync(h, t->nodes->as<uint32_t>() + whir::gpu::tree_words(log_h) - 8,
                                      32, cudaMemcpyDeviceToHost, st),
@@ -530,6 +533,13 @@ int whir_debug_set(unsigned flags) {
   API_BEGIN
   need((flags & ~7u) == 0, "unknown debug flags");
   whir::set_debug(flags);
+  API_END
+}
+
+int whir_debug_expire_waits(whir_ctx *ctx, int on) {
+  API_BEGIN
+  need(ctx != nullptr, "null context");
+  ctx->ctx.expire_waits(on != 0);
   API_END
 }
 

@@ -50,6 +50,14 @@ bool dft_tune_valid(int log_h, DftTune t);
 // (16-byte aligned buffers), so the two-pass split does not apply
 bool dft_coset_one_pass(int log_h, size_t h_in, size_t width);
 
+// The tensor-core hash kernels bound their waits for the matrix unit: one that
+// runs out (p2_tensor.cuh) sets *error (pinned host memory), and what its
+// kernel writes is not valid.  expire: every wait counts as run out.
+struct WaitReport {
+  unsigned int *error = nullptr;
+  bool expire = false;
+};
+
 // ---- kernel launches issued by this library (all contexts), for reporting ----
 unsigned long long launch_count();
 void count_launches(unsigned n);
@@ -67,13 +75,14 @@ cudaError_t dft_batch(const uint32_t *in, size_t h_in, size_t width, int log_h, 
 // ---- Merkle (crates/merkle/src/poseidon_packed.rs) ----
 // leaf digests: PaddingFreeSponge<P24, 24, 16, 8> over each row of row_len words
 cudaError_t hash_rows(const uint32_t *rows, size_t n_rows, int row_len, uint32_t *digests,
-                      cudaStream_t st);
+                      cudaStream_t st, const WaitReport &report);
 // all levels above the leaves: level l+1 node i = C(level l node i, node i + n/2)
 // nodes: level 0 (2^log_h digests) first, then each level in turn
 // host_root (optional, device-writable host memory): the root is also written
 // there, and then seq to *flag (when flag is set)
-cudaError_t build_tree(uint32_t *nodes, int log_h, cudaStream_t st, uint32_t *host_root = nullptr,
-                       unsigned int *flag = nullptr, unsigned int seq = 0);
+cudaError_t build_tree(uint32_t *nodes, int log_h, cudaStream_t st, const WaitReport &report,
+                       uint32_t *host_root = nullptr, unsigned int *flag = nullptr,
+                       unsigned int seq = 0);
 // per query: the leaf row then log_h sibling digests bottom-up
 cudaError_t gather_openings(const uint32_t *rows, int row_len, const uint32_t *nodes, int log_h,
                             const uint32_t *idx, int n, uint32_t *out, cudaStream_t st);
@@ -267,7 +276,8 @@ cudaError_t interleave_rows(const uint32_t *src, size_t rows, size_t w, int batc
                             cudaStream_t st);
 // the batched tree over batch * 2^log_h leaves up to the instances' roots:
 // level l (batch 2^(log_h - l) nodes) at batch * level_offset_words(log_h, l)
-cudaError_t build_tree_batch(uint32_t *nodes, int log_h, int batch, cudaStream_t st);
+cudaError_t build_tree_batch(uint32_t *nodes, int log_h, int batch, cudaStream_t st,
+                             const WaitReport &report);
 // per query q: instance inst[q], index idx[q] of its codeword; out + q (row_len
 // + 8 log_h) gets the row then log_h sibling digests bottom-up
 cudaError_t gather_openings_batch(const uint32_t *rows, int row_len, const uint32_t *nodes,

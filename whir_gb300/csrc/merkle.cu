@@ -349,10 +349,10 @@ cudaError_t verify_paths(const PathDesc *d, const uint32_t *words, const uint32_
 }
 
 cudaError_t hash_rows(const uint32_t *rows, size_t n_rows, int row_len, uint32_t *digests,
-                      cudaStream_t st) {
+                      cudaStream_t st, const WaitReport &report) {
   if (n_rows == 0) return cudaSuccess;
   if (leaves_on_tensor(n_rows, row_len) && ((uintptr_t)digests & 15) == 0) {
-    hash_rows_tensor(rows, n_rows, row_len, digests, st);
+    hash_rows_tensor(rows, n_rows, row_len, digests, st, report);
     count_launches(1);
     return cudaGetLastError();
   }
@@ -397,9 +397,10 @@ __global__ void __launch_bounds__(128, 6) compress_level(const uint32_t *__restr
 }
 
 // one level of a tree: `half` nodes from the 2 half nodes at src
-static void launch_level(const uint32_t *src, uint32_t *dst, size_t half, cudaStream_t st) {
+static void launch_level(const uint32_t *src, uint32_t *dst, size_t half, cudaStream_t st,
+                         const WaitReport &report) {
   if (nodes_on_tensor(half)) {
-    compress_level_tensor(src, dst, half, st);
+    compress_level_tensor(src, dst, half, st, report);
   } else {
     const int T = 128;
     launch(compress_level, (unsigned)((half + T - 1) / T), T, 0, st, src, dst, half);
@@ -555,15 +556,15 @@ static int first_split(int S, int split) {
   return std::min(std::max({g, S - 9, 0}), std::min(S, 9));
 }
 
-cudaError_t build_tree(uint32_t *nodes, int log_h, cudaStream_t st, uint32_t *host_root,
-                       unsigned int *flag, unsigned int seq) {
+cudaError_t build_tree(uint32_t *nodes, int log_h, cudaStream_t st, const WaitReport &report,
+                       uint32_t *host_root, unsigned int *flag, unsigned int seq) {
   TreeTune tune = tree_tune(log_h);
   if (!tree_tune_valid(log_h, tune)) tune = TreeTune();
   int l = 0;
   for (; l < log_h && ((size_t)1 << (log_h - l)) / 2 >= ((size_t)1 << tune.wide_log); l++) {
     size_t half = ((size_t)1 << (log_h - l)) / 2;
     launch_level(nodes + level_offset_words(log_h, l), nodes + level_offset_words(log_h, l + 1),
-                 half, st);
+                 half, st, report);
   }
   // the remaining S = log_h - l steps (S <= wide_log) in up to three launches
   const int S = log_h - l, g = first_split(S, tune.split);
@@ -582,14 +583,15 @@ cudaError_t build_tree(uint32_t *nodes, int log_h, cudaStream_t st, uint32_t *ho
 // Wide levels one thread per node, as build_tree; the remaining S levels up
 // to the instances' roots in two subtree launches: batch 2^g CTAs climb
 // S - g levels, then batch CTAs climb g (each CTA holds at most 512 nodes).
-cudaError_t build_tree_batch(uint32_t *nodes, int log_h, int batch, cudaStream_t st) {
+cudaError_t build_tree_batch(uint32_t *nodes, int log_h, int batch, cudaStream_t st,
+                             const WaitReport &report) {
   if (batch < 1 || log_h < 0 || log_h > 30) return cudaErrorInvalidValue;
   const size_t B = (size_t)batch;
   int l = 0;
   for (; l < log_h && (B << (log_h - l)) / 2 >= ((size_t)1 << 15); l++) {
     size_t half = (B << (log_h - l)) / 2;
     launch_level(nodes + B * level_offset_words(log_h, l),
-                 nodes + B * level_offset_words(log_h, l + 1), half, st);
+                 nodes + B * level_offset_words(log_h, l + 1), half, st, report);
   }
   const int S = log_h - l;
   if (S == 0) return cudaGetLastError();

@@ -43,9 +43,9 @@ __device__ __forceinline__ void load_chunk(const uint32_t *__restrict__ row, int
 template <bool VEC>
 __global__ void __launch_bounds__(p2t_threads<24>, 1)
     hash_rows_tensor_kernel(const uint32_t *__restrict__ rows, size_t n_rows, int row_len,
-                            uint32_t *__restrict__ digests, const Tri tri, unsigned int *err) {
+                            uint32_t *__restrict__ digests, const Tri tri, const WaitReport report) {
   extern __shared__ __align__(128) unsigned char sm[];
-  P2Tile<24> t = p2t_begin<24>(sm, g_tab24, err);
+  P2Tile<24> t = p2t_begin<24>(sm, g_tab24, report);
   pdl_wait();
   const size_t tiles = (n_rows + 127) / 128, step = (size_t)gridDim.x * P2Mat<24>::TILES;
   const int lane_row = threadIdx.x & 127;
@@ -120,14 +120,14 @@ __global__ void __launch_bounds__(p2t_threads<24>, 1)
     }
     tile += step;
   }
-  p2t_end<24>(sm);
+  p2t_end<24>(sm, t, report);
 }
 
 __global__ void __launch_bounds__(p2t_threads<16>, 1)
     compress_level_tensor_kernel(const uint32_t *__restrict__ src, uint32_t *__restrict__ dst,
-                                 size_t half, const Tri tri, unsigned int *err) {
+                                 size_t half, const Tri tri, const WaitReport report) {
   extern __shared__ __align__(128) unsigned char sm[];
-  P2Tile<16> t = p2t_begin<16>(sm, g_tab16, err);
+  P2Tile<16> t = p2t_begin<16>(sm, g_tab16, report);
   pdl_wait();
   const size_t tiles = (half + 127) / 128, step = (size_t)gridDim.x * P2Mat<16>::TILES;
   const int lane_row = threadIdx.x & 127;
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(p2t_threads<16>, 1)
     }
     tile += step;
   }
-  p2t_end<16>(sm);
+  p2t_end<16>(sm, t, report);
 }
 
 Tri tri_of(int width) {
@@ -196,26 +196,28 @@ cudaError_t init_poseidon2_tensor() {
   return e;
 }
 
+unsigned int *tensor_wait_error() { return g_wait_error; }
 bool tensor_wait_failed() {
   return g_wait_error && __atomic_load_n(g_wait_error, __ATOMIC_RELAXED) != 0;
 }
 
 void hash_rows_tensor(const uint32_t *rows, size_t n_rows, int row_len, uint32_t *digests,
-                      cudaStream_t st) {
+                      cudaStream_t st, const WaitReport &report) {
   const bool vec = row_len % 4 == 0 && ((uintptr_t)rows & 15) == 0;
   static const Tri tri = tri_of(24);
   if (vec)
     launch(hash_rows_tensor_kernel<true>, grid_of(n_rows), p2t_threads<24>, p2t_smem<24>(), st, rows,
-           n_rows, row_len, digests, tri, g_wait_error);
+           n_rows, row_len, digests, tri, report);
   else
     launch(hash_rows_tensor_kernel<false>, grid_of(n_rows), p2t_threads<24>, p2t_smem<24>(), st, rows,
-           n_rows, row_len, digests, tri, g_wait_error);
+           n_rows, row_len, digests, tri, report);
 }
 
-void compress_level_tensor(const uint32_t *src, uint32_t *dst, size_t half, cudaStream_t st) {
+void compress_level_tensor(const uint32_t *src, uint32_t *dst, size_t half, cudaStream_t st,
+                           const WaitReport &report) {
   static const Tri tri = tri_of(16);
   launch(compress_level_tensor_kernel, grid_of(half), p2t_threads<16>, p2t_smem<16>(), st, src, dst,
-         half, tri, g_wait_error);
+         half, tri, report);
 }
 
 }  // namespace gpu

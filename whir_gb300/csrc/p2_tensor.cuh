@@ -22,6 +22,7 @@
 // needs 112 columns at least.)  The tables (86 KB at width 24) are read once
 // per CTA.
 #pragma once
+#include "kernels.h"
 #include "launch.cuh"
 #include "p2_matrix.h"
 
@@ -148,6 +149,27 @@ __device__ __forceinline__ int64_t p2t_form(uint32_t b0, uint32_t b1, uint32_t b
 __device__ __forceinline__ uint32_t p2t_low(uint32_t u) { return __byte_perm(u, 0, 0x4140); }
 __device__ __forceinline__ uint32_t p2t_high(uint32_t u) { return __byte_perm(u, 0, 0x4342); }
 
+// bounded wait for a barrier's phase: 2^18 polls, 3.8 us each while nothing
+// arrives, so one second (the bound as a kernel argument costs 0.9% of 2^21
+// rows of 32 words, and so does writing the host's flag in the loop)
+__device__ __forceinline__ bool p2t_wait(uint32_t mbar, uint32_t parity) {
+  uint32_t done = 0;
+  for (int i = 0; i < (1 << 18) && !done; i++)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(mbar), "r"(parity), "r"(1000u)
+        : "memory");
+  return done != 0;
+}
+__device__ __forceinline__ void mma_commit(uint32_t mbar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
+      : "memory");
+}
+
 // One tile of a CTA.  Every member is called by all 128 threads.
 template <int W>
 struct P2Tile {
@@ -157,7 +179,6 @@ struct P2Tile {
   uint32_t tab;    // shared address of the tables, / 16
   uint32_t mbar;   // shared address of the tile's barrier
   uint32_t parity;
-  unsigned int *err;  // host flag: a wait ran out
   int bar;         // named barrier of the tile
   bool issuer;     // this warp issues the tile's matrix instructions
   bool dead;       // a wait ran out: no more waiting
@@ -175,34 +196,17 @@ struct P2Tile {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (elect_one()) {
         issue();
-        asm volatile(
-            "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                mbar)
-            : "memory");
+        mma_commit(mbar);
       }
       __syncwarp();
     }
   }
   // The issuing warp alone polls the barrier and then releases the tile's
-  // other warps.
+  // other warps.  When its wait runs out the tile goes on without waiting, its
+  // results not valid; p2t_end waits for the products and tells the host.
   __device__ __forceinline__ void finish() {
     if (issuer) {
-      if (!dead) {
-        uint32_t done = 0;
-        // bounded: about a second of tries, then the host is told
-        for (int i = 0; i < (1 << 20) && !done; i++)
-          asm volatile(
-              "{\n\t.reg .pred p;\n\t"
-              "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-              "selp.u32 %0, 1, 0, p;\n\t}"
-              : "=r"(done)
-              : "r"(mbar), "r"(parity), "r"(1000u)
-              : "memory");
-        if (!done) {
-          dead = true;
-          *reinterpret_cast<volatile unsigned int *>(err) = 1u;
-        }
-      }
+      if (!dead) dead = !p2t_wait(mbar, parity);
       __syncwarp();
       parity ^= 1u;
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -398,14 +402,14 @@ __device__ __forceinline__ uint32_t p2t_unsigned(int32_t v) {
 }
 
 // A CTA's start and end.  Shared memory: the tables, one barrier per tile,
-// the tensor-memory address.
+// the tensor-memory address, one more barrier per tile for a wait that ran out.
 template <int W>
 constexpr size_t p2t_smem() {
-  return P2Mat<W>::bytes + 8 * (P2Mat<W>::TILES + 1) + 16;
+  return P2Mat<W>::bytes + 8 * (2 * P2Mat<W>::TILES + 1);
 }
 template <int W>
 __device__ __forceinline__ P2Tile<W> p2t_begin(unsigned char *sm, const uint4 *table,
-                                               unsigned int *err) {
+                                               const WaitReport &report) {
   using L = P2Mat<W>;
   static_assert(L::bytes % 16 == 0, "table copy");
   uint64_t *bars = reinterpret_cast<uint64_t *>(sm + L::bytes);
@@ -437,17 +441,33 @@ __device__ __forceinline__ P2Tile<W> p2t_begin(unsigned char *sm, const uint4 *t
   t.tab = smem_addr(sm) >> 4;
   t.mbar = smem_addr(bars + tile);
   t.parity = 0;
-  t.err = err;
   t.bar = 1 + tile;
   t.issuer = warp == (tile & 3);  // one issuer per scheduler
-  t.dead = false;
+  t.dead = report.expire;
   // the constants' operands, and zeros where internal outputs 20.. will be
   const uint32_t c[8] = {0, 0, 0, 0, 0, 0, P2M_CONST0, P2M_CONST1};
   tm_st8(t.row + L::COL_C, c);
   return t;
 }
 template <int W>
-__device__ __forceinline__ void p2t_end(unsigned char *sm) {
+__device__ __forceinline__ void p2t_end(unsigned char *sm, const P2Tile<W> &t,
+                                        const WaitReport &report) {
+  // a tile that gave up a wait: the host is told, and its products end before
+  // the columns are freed (a commit covers all that the thread has issued)
+  if (t.issuer && __any_sync(0xffffffffu, t.dead)) {
+    *reinterpret_cast<volatile unsigned int *>(report.error) = 1u;
+    __threadfence_system();
+    const uint32_t bar = t.mbar + 8 * (P2Mat<W>::TILES + 1);
+    if (elect_one()) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      mma_commit(bar);
+    }
+    __syncwarp();
+    p2t_wait(bar, 0);
+    __syncwarp();
+  }
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();

@@ -141,6 +141,9 @@ void *Context::pinned(size_t bytes) {
   }
   return pinned_;
 }
+gpu::WaitReport Context::wait_report() const {
+  return {gpu::tensor_wait_error(), expire_waits_};
+}
 // a kernel gave up a bounded wait: what it wrote is not valid
 static void check_kernel_waits() {
   if (gpu::tensor_wait_failed()) throw WhirError(-2, "a hash kernel's wait ran out");
@@ -280,13 +283,15 @@ void encode_commit(Context &ctx, const uint32_t *src, int k, int rate, int foldi
     ctx.prof_end(Context::K_DFT, 4.0 * (double)(h_in * width + rows * width));
   }
   ctx.prof_begin(Context::K_LEAF);
-  cuda_check(gpu::hash_rows(codeword, rows, (int)width, nodes, st), "hash_rows");
+  cuda_check(gpu::hash_rows(codeword, rows, (int)width, nodes, st, ctx.wait_report()),
+             "hash_rows");
   ctx.prof_end(Context::K_LEAF, 4.0 * (double)(rows * width + rows * 8));
   // the last tree launch writes the root straight into pinned host memory
   uint32_t *h = (uint32_t *)ctx.pinned(64);
   unsigned int seq = ctx.next_seq();
   ctx.prof_begin(Context::K_TREE);
-  cuda_check(gpu::build_tree(nodes, log_h, st, h, ctx.flag(), seq), "build_tree");
+  cuda_check(gpu::build_tree(nodes, log_h, st, ctx.wait_report(), h, ctx.flag(), seq),
+             "build_tree");
   ctx.prof_end(Context::K_TREE, 32.0 * (double)(2 * rows - 2 + rows - 1));
   if (log_h == 0) {  // a single leaf is the root; no tree launch ran
     cuda_check(copy_async(ctx, h, nodes, 32, cudaMemcpyDeviceToHost), "root copy");

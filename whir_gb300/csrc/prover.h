@@ -132,6 +132,9 @@ class Context {
   unsigned int *flag() const { return flag_; }
   unsigned int next_seq() { return seq_ = seq_ + 1 ? seq_ + 1 : 1; }
   void wait_flag(unsigned int seq);
+  // where this context's hash kernels report a wait that ran out
+  gpu::WaitReport wait_report() const;
+  void expire_waits(bool on) { expire_waits_ = on; }
   // per-kernel-class CUDA-event timing on this stream
   // kernel classes timed with events, and K_SYNC: host time blocked in sync()
   enum Klass { K_DFT = 0, K_LEAF = 1, K_TREE = 2, K_SUMCHECK = 3, K_SYNC = 4, K_NCLASS = 5 };
@@ -155,6 +158,7 @@ class Context {
   cudaEvent_t block_ev_ = nullptr;
   unsigned int *flag_ = nullptr;
   unsigned int seq_ = 0;
+  bool expire_waits_ = false;
   cudaStream_t stream_ = nullptr;
   cudaStream_t streams_[2] = {nullptr, nullptr};  // normal, high priority
   void *pinned_ = nullptr;

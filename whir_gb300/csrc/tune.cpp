@@ -61,7 +61,8 @@ std::string autotune(Context &ctx, int lo, int hi) {
           if (h <= wl && wl != base.wide_log) continue;  // wide_log >= h: the same split
           gpu::set_tree_tune(h, t);
           double ms = time_ms(ctx, a, b, [&] {
-            cuda_check(gpu::build_tree(nodes.as<uint32_t>(), h, st), "build_tree");
+            cuda_check(gpu::build_tree(nodes.as<uint32_t>(), h, st, ctx.wait_report()),
+                       "build_tree");
           });
           if (wl == base.wide_log && sp == base.split) base_ms = ms;
           if (ms < best_ms) {
