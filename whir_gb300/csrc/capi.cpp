@@ -144,7 +144,7 @@ int whir_device_alloc(whir_ctx *ctx, size_t bytes, void **out) {
 int whir_device_free(whir_ctx *ctx, void *ptr) {
   API_BEGIN
   need(ctx != nullptr, "null context");
-  ctx->ctx.sync();
+  ctx->ctx.drain();
   whir::cuda_check(cudaFree(ptr), "cudaFree");
   API_END
 }
@@ -255,14 +255,14 @@ int whir_merkle_open(whir_tree *tree, const size_t *idx, size_t n, uint32_t *out
 }
 int whir_merkle_free(whir_tree *tree) {
   API_BEGIN
-  if (tree) {
-    whir_ctx *c = tree->ctx;
-    c->ctx.sync();
+  std::unique_ptr<whir_tree> t(tree);  // released whatever the stream reports
+  if (t) {
+    whir_ctx *c = t->ctx;
+    c->ctx.drain();
     std::lock_guard<std::mutex> lock(c->spare_mu);
-    if (tree->nodes && (!c->spare_nodes || c->spare_nodes->bytes() < tree->nodes->bytes()))
-      c->spare_nodes = std::move(tree->nodes);
+    if (t->nodes && (!c->spare_nodes || c->spare_nodes->bytes() < t->nodes->bytes()))
+      c->spare_nodes = std::move(t->nodes);
   }
-  delete tree;
   API_END
 }
 

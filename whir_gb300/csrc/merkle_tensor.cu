@@ -1,7 +1,5 @@
 // Leaf hashing and node compression with the tensor-core permutation
 // (p2_tensor.cuh); merkle.cu decides which sizes run here.
-#include <mutex>
-
 #include "kernels.h"
 #include "launch.cuh"
 #include "merkle_tensor.h"
@@ -14,7 +12,6 @@ namespace {
 constexpr int SMS = 152;
 __device__ uint4 g_tab16[P2Mat<16>::bytes / 16];
 __device__ uint4 g_tab24[P2Mat<24>::bytes / 16];
-unsigned int *g_wait_error;  // pinned, set by a kernel whose wait ran out
 
 struct Tri {
   int32_t v[4];
@@ -178,15 +175,7 @@ unsigned grid_of(size_t n) {
 }  // namespace
 
 cudaError_t init_poseidon2_tensor() {
-  static std::mutex mu;
-  std::lock_guard<std::mutex> lock(mu);
-  cudaError_t e = cudaSuccess;
-  if (!g_wait_error) {
-    e = cudaHostAlloc(&g_wait_error, 64, cudaHostAllocPortable);
-    if (e != cudaSuccess) return e;
-    *g_wait_error = 0;
-  }
-  e = cudaMemcpyToSymbol(g_tab16, p2_tables(16).halves.data(), P2Mat<16>::bytes);
+  cudaError_t e = cudaMemcpyToSymbol(g_tab16, p2_tables(16).halves.data(), P2Mat<16>::bytes);
   if (e == cudaSuccess)
     e = cudaMemcpyToSymbol(g_tab24, p2_tables(24).halves.data(), P2Mat<24>::bytes);
   const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
@@ -194,11 +183,6 @@ cudaError_t init_poseidon2_tensor() {
   if (e == cudaSuccess) e = cudaFuncSetAttribute(hash_rows_tensor_kernel<false>, a, p2t_smem<24>());
   if (e == cudaSuccess) e = cudaFuncSetAttribute(compress_level_tensor_kernel, a, p2t_smem<16>());
   return e;
-}
-
-unsigned int *tensor_wait_error() { return g_wait_error; }
-bool tensor_wait_failed() {
-  return g_wait_error && __atomic_load_n(g_wait_error, __ATOMIC_RELAXED) != 0;
 }
 
 void hash_rows_tensor(const uint32_t *rows, size_t n_rows, int row_len, uint32_t *digests,

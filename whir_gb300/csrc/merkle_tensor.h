@@ -9,15 +9,12 @@
 namespace whir {
 namespace gpu {
 
-cudaError_t init_poseidon2_tensor();  // per device: tables, attributes, the wait flag
+cudaError_t init_poseidon2_tensor();  // per device: tables, attributes
 // digests on a 16-byte boundary
 void hash_rows_tensor(const uint32_t *rows, size_t n_rows, int row_len, uint32_t *digests,
                       cudaStream_t st, const WaitReport &report);
 void compress_level_tensor(const uint32_t *src, uint32_t *dst, size_t half, cudaStream_t st,
                            const WaitReport &report);
-// a kernel's bounded wait ran out (its results are not valid)
-unsigned int *tensor_wait_error();
-bool tensor_wait_failed();
 
 }  // namespace gpu
 }  // namespace whir

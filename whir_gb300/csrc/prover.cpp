@@ -2,7 +2,6 @@
 #include "prover.h"
 #include "debug.h"
 #include "host_math.h"
-#include "merkle_tensor.h"
 #include "svo_host.h"
 #include "verifier.h"
 
@@ -115,7 +114,7 @@ Context::Context(int device) : device_(device) {
   stream_ = streams_[0];
   cuda_check(gpu::init_device_tables(), "device tables");
   cuda_check(cudaMallocHost(&flag_, 64), "cudaMallocHost");
-  *flag_ = 0;
+  flag_[0] = flag_[WAIT_ERROR] = 0;
 }
 Context::~Context() {
   cudaSetDevice(device_);
@@ -141,18 +140,17 @@ void *Context::pinned(size_t bytes) {
   }
   return pinned_;
 }
-gpu::WaitReport Context::wait_report() const {
-  return {gpu::tensor_wait_error(), expire_waits_};
-}
-// a kernel gave up a bounded wait: what it wrote is not valid
-static void check_kernel_waits() {
-  if (gpu::tensor_wait_failed()) throw WhirError(-2, "a hash kernel's wait ran out");
+void Context::check_waits() {
+  if (!__atomic_load_n(flag_ + WAIT_ERROR, __ATOMIC_RELAXED)) return;
+  drain();  // kernels launched before this point report into this error
+  __atomic_store_n(flag_ + WAIT_ERROR, 0u, __ATOMIC_RELAXED);
+  throw WhirError(-2, "a hash kernel's wait ran out");
 }
 void Context::wait_stream() {
-  wait_stream_done();
-  check_kernel_waits();
+  drain();
+  check_waits();
 }
-void Context::wait_stream_done() {
+void Context::drain() {
   if (!yield_) {
     cuda_check(cudaStreamSynchronize(stream_), "stream sync");
     return;
@@ -194,7 +192,7 @@ void Context::wait_flag(unsigned int seq) {
     }
     if (yield_) std::this_thread::yield();
   }
-  check_kernel_waits();
+  check_waits();
   if (prof_on(K_SYNC)) {
     acc_ms_[K_SYNC] +=
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();

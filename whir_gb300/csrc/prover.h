@@ -122,6 +122,8 @@ class Context {
   void set_high_priority(bool on);
   void *pinned(size_t bytes);  // staging for D2H results and H2D arguments
   void sync();
+  // waits for the stream only: neither reports nor takes an error of its kernels
+  void drain();
   // Waiting for the stream: a blocking synchronise (lowest latency, keeps a
   // core busy), or a short poll with yields followed by a sleep on a
   // blocking-sync event, so that many worker threads can share the host cores.
@@ -133,7 +135,7 @@ class Context {
   unsigned int next_seq() { return seq_ = seq_ + 1 ? seq_ + 1 : 1; }
   void wait_flag(unsigned int seq);
   // where this context's hash kernels report a wait that ran out
-  gpu::WaitReport wait_report() const;
+  gpu::WaitReport wait_report() const { return {flag_ + WAIT_ERROR, expire_waits_}; }
   void expire_waits(bool on) { expire_waits_ = on; }
   // per-kernel-class CUDA-event timing on this stream
   // kernel classes timed with events, and K_SYNC: host time blocked in sync()
@@ -151,8 +153,11 @@ class Context {
   unsigned long long d2h_bytes() const { return d2h_bytes_; }
 
  private:
-  void wait_stream();       // and fails if a kernel gave up a bounded wait
-  void wait_stream_done();
+  static constexpr int WAIT_ERROR = 8;  // its word behind flag_
+  void wait_stream();  // drain() and check_waits()
+  // fails, once, if a kernel of this stream gave up a bounded wait: what was
+  // written since is not valid
+  void check_waits();
   int device_;
   bool yield_ = false;
   cudaEvent_t block_ev_ = nullptr;

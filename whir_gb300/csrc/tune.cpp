@@ -75,6 +75,7 @@ std::string autotune(Context &ctx, int lo, int hi) {
                h, best.wide_log, best.split, best_ms, base_ms);
       rep += line;
     }
+    ctx.sync();  // and a tree kernel that gave up a wait is reported here
     // two-pass DFTs at the WHIR shapes: base rows of 16 words from a quarter
     // of the rows, extension rows of 64 words from a 32nd
     for (size_t width : {(size_t)16, (size_t)64}) {
