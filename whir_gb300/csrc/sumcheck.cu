@@ -10,6 +10,7 @@
 // bit for bit.
 #include "kernels.h"
 #include "launch.cuh"
+#include "point_plan.h"
 
 namespace whir {
 namespace gpu {
@@ -473,10 +474,7 @@ cudaError_t compress_hi_batch(const uint32_t *poly, int k, int ks, const E4 *eq_
 
 cudaError_t compress_hi_point(const uint32_t *poly, int k, const Point &z,
                               unsigned long long *acc, cudaStream_t st, const Publish &pub) {
-  // blocks of 4096 words where the polynomial has them (the pipelined kernel);
-  // shorter ones otherwise, so that a small polynomial still has several CTAs
-  const int ks = k - z.k;
-  const int s_lo = ks >= 2 && k >= 12 ? 12 - ks : z.k < 8 ? z.k : 8;
+  const int ks = k - z.k, s_lo = compress_hi_point_low(k, ks);
   return compress_hi_launch(poly, k, ks, &z, nullptr, s_lo, nullptr, acc, 1, HiStrides(), st, pub);
 }
 
