@@ -590,8 +590,9 @@ __device__ __forceinline__ void dif_last_v(const uint4 *tile, const TW &tw, int 
   }
 }
 
-// MINB: CTAs per SM the registers must allow; tiles of more than 48 KB fit
-// three per SM by shared memory, so they take up to 80 registers a thread.
+// MINB: CTAs per SM the registers must allow: four, or three (up to 80 registers
+// a thread) for tiles of more than 48 KB, which fit three per SM by shared
+// memory, and for launches of no more CTAs than that.
 // MODE: S mod 3 for S >= 6, 3 for S = 4 and 5, so that a kernel holds only the
 // steps of its sizes (one kernel for all spilled at 80 registers).
 // Bound by the latency of the global steps: with the S mod 3 stages first a
@@ -599,10 +600,12 @@ __device__ __forceinline__ void dif_last_v(const uint4 *tile, const TW &tw, int 
 // and last it has eight, and the stores of a row follow its twiddle at once.
 // 2^21 rows of 64 words from 2^16 636 -> 607 us, 2^20 of 16 from 2^18
 // 93.7 -> 86.2 us, 2^20 of 64 from 2^12 292 -> 275 us, 2^19 of 20 from
-// 200003 79.3 -> 72.0 us; sizes of one wave within 0.4 us either way.
+// 200003 79.3 -> 72.0 us.
 // HOIST (twiddles of a thread's tasks loaded once) spills at the 64 registers
-// of four CTAs (2^20 rows of 16 words 87.6 us with it), so only the three-CTA
-// tiles take it.
+// of four CTAs (2^20 rows of 16 words 87.6 us with it), so only MINB = 3 takes
+// it.  Few CTAs wait for their own steps and not for a slot: MINB = 3 against 4
+// there, 2^9 rows of 64 words 5.8 against 6.9 us, 2^6 4.8 / 5.3, 2^13 from 2^9
+// 11.1 / 12.4; at 1024 CTAs (2^13 of 512 from 2^9) 19.4 / 17.8.
 template <int C, int MINB, int MODE>
 __global__ void __launch_bounds__(256, MINB) dft_tile_v2(const uint32_t *__restrict__ in,
                                                    uint32_t *__restrict__ out, int S, int lg,
@@ -676,12 +679,12 @@ static cudaError_t launch_tile_v(const uint32_t *in, uint32_t *out, int S, size_
   dim3 grid((unsigned)(width / C), (unsigned)(n_outer >> lg));
   if (S >= 4) {
     // above 48 KB: sub-transforms of 2^12 rows, and of 2^11 at C = 8
-    static const decltype(&dft_tile_v2<C, 4, 0>) narrow[4] = {
+    static const decltype(&dft_tile_v2<C, 4, 0>) four[4] = {
         dft_tile_v2<C, 4, 0>, dft_tile_v2<C, 4, 1>, dft_tile_v2<C, 4, 2>, dft_tile_v2<C, 4, 3>};
-    const auto kernel = rows * C * 4 <= (48u << 10) ? narrow[S < 6 ? 3 : S % 3]
-                        : S == 12                   ? dft_tile_v2<C, 3, 0>
-                                                    : dft_tile_v2<C, 3, C == 8 ? 2 : 0>;
-    launch(kernel, grid, threads, rows * C * 4, st, in, out, S, lg, (uint32_t)width,
+    static const decltype(&dft_tile_v2<C, 4, 0>) three[4] = {
+        dft_tile_v2<C, 3, 0>, dft_tile_v2<C, 3, 1>, dft_tile_v2<C, 3, 2>, dft_tile_v2<C, 3, 3>};
+    const bool full = rows * C * 4 <= (48u << 10) && (size_t)grid.x * grid.y > 3 * 152;
+    launch((full ? four : three)[S < 6 ? 3 : S % 3], grid, threads, rows * C * 4, st, in, out, S, lg, (uint32_t)width,
            (uint32_t)rows_valid, (uint32_t)a_in, (uint32_t)b_in, (uint32_t)a_out,
            (uint32_t)b_out, pre_log, tw_log, ix);
   }
