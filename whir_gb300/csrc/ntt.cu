@@ -474,34 +474,35 @@ __device__ __forceinline__ void dif_first_v(uint4 *tile, const TW &tw, int rows_
     const int j = rest & (q - 1), blk = rest >> lq;
     const int base = blk * 2 * H + j;
     uint4 v[T];
-    // the task's rows lie in one sub-transform (T q = 2^S rows), so their
-    // coset pre-twiddles w^(o' i) with i = i0 + t q form a geometric
-    // sequence: two table lookups, then one product per row
-    uint32_t ptw = 0, pstep = 0;
-    if (pre_log) {
-      const uint32_t o = o0 + (uint32_t)(base >> S), i0 = (uint32_t)(base & (n - 1));
-      const uint32_t oo = o >> ix.pre_shift;
-      ptw = root_pow(((oo * i0) & pmask) << (24 - pre_log));
-      pstep = root_pow(((oo * (uint32_t)q) & pmask) << (24 - pre_log));
-    }
 #pragma unroll
     for (int t = 0; t < T; t++) {
       const int r = base + t * q;
       const uint32_t o = o0 + (uint32_t)(r >> S), i = (uint32_t)(r & (n - 1));
       const uint32_t row = (o & ix.in_mask) * a_in + i * b_in;
       v[t] = make_uint4(0, 0, 0, 0);
-      if (row < rows_valid) {
-        // rows read once bypass the L1 (it keeps the twiddles); coset
-        // transforms (pre_log > 0) read every input row once per coset, so
-        // theirs stay cached
-        if (pre_log) {
-          v[t] = __ldg(in4 + row * wv + v0 + c);
-          v[t] = mul4(v[t], ptw);
-        } else {
-          v[t] = __ldcg(in4 + row * wv + v0 + c);
-        }
+      // rows read once bypass the L1 (it keeps the twiddles); coset
+      // transforms (pre_log > 0) read every input row once per coset, so
+      // theirs stay cached
+      if (row < rows_valid)
+        v[t] = pre_log ? __ldg(in4 + row * wv + v0 + c) : __ldcg(in4 + row * wv + v0 + c);
+    }
+    // The task's rows lie in one sub-transform (T q = 2^S rows), so their
+    // coset pre-twiddles w^(o' i) with i = i0 + t q form a geometric
+    // sequence: two table lookups, then one product per row.  A pass of its
+    // own over the rows, after all their loads are on the way: with a row's
+    // product behind its load the T loads waited for one another (us, 2^14 rows
+    // of 16 words from 2^9 9.9 -> 6.5, from 2^7 9.4 -> 6.5, 2^16 of 128 words
+    // from 2^11 39.0 -> 32.9, from 2^8 26.8 -> 24.7).
+    if (pre_log) {
+      const uint32_t o = o0 + (uint32_t)(base >> S), i0 = (uint32_t)(base & (n - 1));
+      const uint32_t oo = o >> ix.pre_shift;
+      uint32_t ptw = root_pow(((oo * i0) & pmask) << (24 - pre_log));
+      const uint32_t pstep = root_pow(((oo * (uint32_t)q) & pmask) << (24 - pre_log));
+#pragma unroll
+      for (int t = 0; t < T; t++) {
+        v[t] = mul4(v[t], ptw);
+        if (t + 1 < T) ptw = kb::mul(ptw, pstep);
       }
-      if (pre_log && t + 1 < T) ptw = kb::mul(ptw, pstep);
     }
 #pragma unroll
     for (int st = 0; st < R; st++) {
@@ -604,8 +605,9 @@ __device__ __forceinline__ void dif_last_v(const uint4 *tile, const TW &tw, int 
 // HOIST (twiddles of a thread's tasks loaded once) spills at the 64 registers
 // of four CTAs (2^20 rows of 16 words 87.6 us with it), so only MINB = 3 takes
 // it.  Few CTAs wait for their own steps and not for a slot: MINB = 3 against 4
-// there, 2^9 rows of 64 words 5.8 against 6.9 us, 2^6 4.8 / 5.3, 2^13 from 2^9
-// 11.1 / 12.4; at 1024 CTAs (2^13 of 512 from 2^9) 19.4 / 17.8.
+// there, 2^9 rows of 64 words 5.3 against 6.8 us, 2^6 4.3 / 5.3, 2^13 from 2^9
+// 7.0 / 8.5; at 512 CTAs (2^13 of 256) from 2^6 8.6 / 8.8, from 2^8 10.1 / 10.0,
+// at 1024 13.3 / 12.9 and 15.7 / 15.3.
 template <int C, int MINB, int MODE>
 __global__ void __launch_bounds__(256, MINB) dft_tile_v2(const uint32_t *__restrict__ in,
                                                    uint32_t *__restrict__ out, int S, int lg,
@@ -721,8 +723,9 @@ static cudaError_t tile_any(const uint32_t *in, uint32_t *out, int S, size_t wid
                             size_t a_out, size_t b_out, int pre_log, int tw_log, cudaStream_t st) {
   const bool aligned = (((uintptr_t)in | (uintptr_t)out) & 15) == 0;
   // Slices of 8 columns read whole 32-byte sectors, but where they leave half
-  // of the SMs idle twice as many of 4 finish sooner (us, 16 columns: 2^11 rows
-  // 9.2 -> 6.8, 2^12 from 2^11 12.7 -> 8.6, 2^10 5.3 -> 4.8).
+  // of the SMs idle twice as many of 4 finish sooner (us of a lone cold launch, 16
+  // columns, 8 / 4 a slice: 2^11 rows 11.7 / 7.8, 2^12 from 2^11 13.3 / 9.6, 2^10
+  // 6.9 / 6.4, 2^14 from 2^8 7.0 / 6.6; above, 2^14 of 64 from 2^8 7.4 / 8.6).
   int lg = 0;
   while (S + lg < 10 && ((size_t)2 << lg) <= n_outer) lg++;
   const bool few = (width / 8) * (n_outer >> lg) <= 76;
@@ -751,8 +754,9 @@ static int ceil_log2(size_t x) {
   return l;
 }
 // 2^12-row tiles follow each other's steps for 15 us however few they are; up
-// to 64 of them two passes of smaller tiles are faster (us, one pass and two:
-// 2^14 rows of 16 words 15.1 / 11.0, of 64 15.6 / 11.6, 2^15 of 64 15.8 / 16.3).
+// to 64 of them two passes of smaller tiles are faster (us, cold, one pass and
+// two: 2^14 rows of 16 words 15.9 / 12.2, of 64 17.7 / 16.8, 2^15 of 64 18.0 /
+// 19.2).
 static bool coset12_one_pass(int log_h, size_t width) {
   return width % 4 == 0 && ((width / 4) << (log_h - 12)) > 64;
 }
