@@ -290,15 +290,7 @@ int whir_compress_hi(whir_ctx *ctx, const uint32_t *poly, int k, const uint32_t 
   cudaStream_t st = ctx->ctx.stream();
   size_t words = (size_t)4 << ks;
   unsigned long long *a = acc_buf(ctx, words);
-  if (k <= 28) {
-    whir::cuda_check(whir::gpu::compress_hi_point(poly, k, z, a, st), "compress_hi");
-  } else {  // its CTAs' high tables would outgrow shared memory
-    int s_lo = kz < 10 ? kz : 10;
-    ctx->eq.reserve(sizeof(E4) * (((size_t)1 << s_lo) + ((size_t)1 << (kz - s_lo))));
-    E4 *lo = ctx->eq.as<E4>(), *hi = lo + ((size_t)1 << s_lo);
-    whir::cuda_check(whir::gpu::eq_split(z, s_lo, kb::e_one(), lo, hi, st), "eq_split");
-    whir::cuda_check(whir::gpu::compress_hi(poly, k, ks, lo, s_lo, hi, a, st), "compress_hi");
-  }
+  whir::cuda_check(whir::gpu::compress_hi_point(poly, k, z, a, st), "compress_hi");
   read_acc(ctx, a, words, out);
   API_END
 }
@@ -324,18 +316,8 @@ int whir_eval_ext(whir_ctx *ctx, const uint32_t *poly, int k, const uint32_t *po
   whir::gpu::Point z = point_in(point, k);
   cudaStream_t st = ctx->ctx.stream();
   unsigned long long *a = acc_buf(ctx, 4);
-  if (k <= 26) {
-    whir::cuda_check(whir::gpu::eval_ext_point(reinterpret_cast<const E4 *>(poly), z, a, st),
-                     "eval_ext");
-  } else {  // its CTAs' high tables would outgrow shared memory
-    int s_lo = 10;
-    ctx->eq.reserve(sizeof(E4) * (((size_t)1 << s_lo) + ((size_t)1 << (k - s_lo))));
-    E4 *lo = ctx->eq.as<E4>(), *hi = lo + ((size_t)1 << s_lo);
-    whir::cuda_check(whir::gpu::eq_split(z, s_lo, kb::e_one(), lo, hi, st), "eq_split");
-    whir::cuda_check(
-        whir::gpu::eval_ext(reinterpret_cast<const E4 *>(poly), k, lo, s_lo, hi, a, st),
-        "eval_ext");
-  }
+  whir::cuda_check(whir::gpu::eval_ext_point(reinterpret_cast<const E4 *>(poly), z, a, st),
+                   "eval_ext");
   read_acc(ctx, a, 4, out);
   API_END
 }

@@ -185,11 +185,8 @@ cudaError_t sumcheck_round(const kb::E4 *p_in, const kb::E4 *w_in, size_t n_in, 
                            kb::E4 r, kb::E4 *p_out, kb::E4 *w_out, bool coeffs,
                            unsigned long long *acc, cudaStream_t st,
                            const Publish &pub = Publish());
-// <eq(z), poly> for an extension poly (SplitEq::eval_ext, eq.rs:179-250) -> acc u64[4]
-cudaError_t eval_ext(const kb::E4 *poly, int k, const kb::E4 *eq_lo, int s_lo,
-                     const kb::E4 *eq_hi, unsigned long long *acc, cudaStream_t st,
-                     const Publish &pub = Publish());
-// the same with the tables formed by the kernel (z.k variables)
+// <eq(z), poly> for an extension poly of z.k variables (SplitEq::eval_ext,
+// eq.rs:179-250) -> acc u64[4]; the eq tables are formed by the kernel
 cudaError_t eval_ext_point(const kb::E4 *poly, const Point &z, unsigned long long *acc,
                            cudaStream_t st, const Publish &pub = Publish());
 // <a, b> of two extension arrays of n elements -> acc u64[4] (debug checks)
@@ -260,7 +257,8 @@ cudaError_t sumcheck_round_batch(const kb::E4 *p_in, const kb::E4 *w_in, size_t 
                                  const kb::E4 *r_b, kb::E4 *p_out, kb::E4 *w_out, bool coeffs,
                                  unsigned long long *acc, size_t acc_stride, int batch,
                                  cudaStream_t st, const Publish &pub = Publish());
-// instance y: poly + y 2^k, tables at y tab_stride, sum at acc + 4 y
+// the same from eq tables: instance y: poly + y 2^k, tables at y tab_stride, sum
+// at acc + 4 y
 cudaError_t eval_ext_batch(const kb::E4 *poly, int k, const kb::E4 *eq_lo, int s_lo,
                            const kb::E4 *eq_hi, size_t tab_stride, int batch,
                            unsigned long long *acc, cudaStream_t st,

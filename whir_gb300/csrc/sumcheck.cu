@@ -432,11 +432,9 @@ cudaError_t compress_hi(const uint32_t *poly, int k, int ks, const E4 *eq_lo, in
   return compress_hi_batch(poly, k, ks, eq_lo, s_lo, eq_hi, acc, 1, HiStrides(), st, pub);
 }
 
-// z: PT (its own tables), one instance; else the tables at eq_lo and eq_hi
-static cudaError_t compress_hi_launch(const uint32_t *poly, int k, int ks, const Point *z,
-                                      const E4 *eq_lo, int s_lo, const E4 *eq_hi,
-                                      unsigned long long *acc, int batch, const HiStrides &sd,
-                                      cudaStream_t st, const Publish &pub) {
+cudaError_t compress_hi_batch(const uint32_t *poly, int k, int ks, const E4 *eq_lo, int s_lo,
+                              const E4 *eq_hi, unsigned long long *acc, int batch,
+                              const HiStrides &sd, cudaStream_t st, const Publish &pub) {
   if ((1 << ks) > CH_T || k < ks + s_lo || batch < 1 || batch > 65535)
     return cudaErrorInvalidValue;
   size_t n_hi = (size_t)1 << (k - ks - s_lo);
@@ -445,37 +443,22 @@ static cudaError_t compress_hi_launch(const uint32_t *poly, int k, int ks, const
   const size_t per = ((size_t)152 * (pipe ? 3 : 4) + batch - 1) / batch;
   dim3 grid((unsigned)(n_hi < per ? n_hi : per), (unsigned)batch);
   size_t smem = ((size_t)1 << s_lo) * sizeof(E4) + ((size_t)4 << ks) * 8;
-  if (z) {
-    smem += sizeof(E4) * (64 + (n_hi + grid.x - 1) / grid.x);
-    if (s_lo > 10 || z->k != k - ks || batch != 1 || smem > 48 * 1024)
-      return cudaErrorInvalidValue;
-    if (pipe)
-      launch(compress_hi_pipe_kernel<true>, grid, CH_T, smem, st, poly, k, ks, *z, eq_lo, s_lo,
-             eq_hi, acc, pub, sd);
-    else
-      launch(compress_hi_kernel<true>, grid, CH_T, smem, st, poly, k, ks, *z, eq_lo, s_lo, eq_hi,
-             acc, pub, sd);
-  } else if (pipe) {
-    launch(compress_hi_pipe_kernel<false>, grid, CH_T, smem, st, poly, k, ks, Point(), eq_lo, s_lo,
-           eq_hi, acc, pub, sd);
-  } else {
-    launch(compress_hi_kernel<false>, grid, CH_T, smem, st, poly, k, ks, Point(), eq_lo, s_lo,
-           eq_hi, acc, pub, sd);
-  }
+  launch(pipe ? compress_hi_pipe_kernel<false> : compress_hi_kernel<false>, grid, CH_T, smem, st,
+         poly, k, ks, Point(), eq_lo, s_lo, eq_hi, acc, pub, sd);
   count_launches(1);
   return cudaGetLastError();
 }
 
-cudaError_t compress_hi_batch(const uint32_t *poly, int k, int ks, const E4 *eq_lo, int s_lo,
-                              const E4 *eq_hi, unsigned long long *acc, int batch,
-                              const HiStrides &sd, cudaStream_t st, const Publish &pub) {
-  return compress_hi_launch(poly, k, ks, nullptr, eq_lo, s_lo, eq_hi, acc, batch, sd, st, pub);
-}
-
 cudaError_t compress_hi_point(const uint32_t *poly, int k, const Point &z,
                               unsigned long long *acc, cudaStream_t st, const Publish &pub) {
-  const int ks = k - z.k, s_lo = compress_hi_point_low(k, ks);
-  return compress_hi_launch(poly, k, ks, &z, nullptr, s_lo, nullptr, acc, 1, HiStrides(), st, pub);
+  const int ks = k - z.k;
+  if (ks < 0 || (1 << ks) > CH_T || z.k < 0 || z.k > MAX_VARS) return cudaErrorInvalidValue;
+  const int s_lo = compress_hi_point_low(k, ks);
+  const PointLaunch l = compress_hi_point_launch(k, ks);
+  launch(ks + s_lo == 12 ? compress_hi_pipe_kernel<true> : compress_hi_kernel<true>, l.ctas, CH_T,
+         l.smem, st, poly, k, ks, z, nullptr, s_lo, nullptr, acc, pub, HiStrides());
+  count_launches(1);
+  return cudaGetLastError();
 }
 
 // compress_lo: out[i] = sum_j eq(rs)[j] * P[i * 2^ks + j].  Batched:
@@ -1165,11 +1148,6 @@ cudaError_t eval_ext_batch(const E4 *poly, int k, const E4 *eq_lo, int s_lo, con
   return cudaGetLastError();
 }
 
-cudaError_t eval_ext(const E4 *poly, int k, const E4 *eq_lo, int s_lo, const E4 *eq_hi,
-                     unsigned long long *acc, cudaStream_t st, const Publish &pub) {
-  return eval_ext_batch(poly, k, eq_lo, s_lo, eq_hi, 0, 1, acc, st, pub);
-}
-
 // The same of one instance with its tables formed here: thread t holds entries
 // t of its CTA's blocks of 256, so its own low entry is one factor at the end.
 template <bool VEC>
@@ -1206,14 +1184,11 @@ cudaError_t eval_ext_point(const E4 *poly, const Point &z, unsigned long long *a
                            cudaStream_t st, const Publish &pub) {
   const int k = z.k;
   if (k < 0 || k > MAX_VARS) return cudaErrorInvalidValue;
-  const size_t n_hi = k < 8 ? 1 : (size_t)1 << (k - 8);
-  const unsigned grid = (unsigned)(n_hi < 152 * 8 ? n_hi : 152 * 8);
-  const size_t smem = sizeof(E4) * (64 + (n_hi + grid - 1) / grid);
-  if (smem > 48 * 1024) return cudaErrorInvalidValue;
+  const PointLaunch l = eval_ext_point_launch(k);
   if (aligned16(poly))
-    launch(eval_ext_point_kernel<true>, grid, 256, smem, st, poly, k, z, acc, pub);
+    launch(eval_ext_point_kernel<true>, l.ctas, 256, l.smem, st, poly, k, z, acc, pub);
   else
-    launch(eval_ext_point_kernel<false>, grid, 256, smem, st, poly, k, z, acc, pub);
+    launch(eval_ext_point_kernel<false>, l.ctas, 256, l.smem, st, poly, k, z, acc, pub);
   count_launches(1);
   return cudaGetLastError();
 }
