@@ -362,11 +362,11 @@ WHIR_API int whir_compress_hi_noalloc(void *cuda_stream, const uint32_t *poly, i
  * stream (a few hundred ms, up to ~1.5 GB of temporary device memory),
  * installs the fastest process-wide and writes a text report (one line per
  * size) into report.  whir_tune_tree / whir_tune_dft set one choice (tree:
- * levels making >= 2^wide_log nodes run one thread per node, the other S as
- * subtrees in one to three launches, the first of 2^split (split in -1..1)
- * times the default number; DFT: first pass of 2^L1
- * rows, L1 = (log_h + 1) / 2 + l1_bias); whir_tune_reset restores the
- * defaults. ---- */
+ * levels making >= 2^wide_log nodes run over the whole GPU, one launch each,
+ * the other S as subtrees in one to three launches, the first of 2^split (split
+ * in -1..1) times the default number, or of the default number where a subtree
+ * would not fit; DFT: first pass of 2^L1 rows, L1 = (log_h + 1) / 2 + l1_bias);
+ * whir_tune_reset restores the defaults. ---- */
 WHIR_API int whir_autotune(whir_ctx *ctx, int log_h_lo, int log_h_hi, char *report, size_t cap);
 WHIR_API int whir_tune_tree(int log_h, int wide_log, int split);
 WHIR_API int whir_tune_dft(int log_h, size_t width, int l1_bias);

@@ -29,10 +29,11 @@ struct Publish {
 // ---- per-size scheduling choices ----
 // How a tree or a DFT of a given size is split into launches.  Every choice
 // computes the same result; whir::autotune picks them by measurement.
-// Tree: levels that make >= 2^wide_log nodes run one thread per node; the
-// remaining S levels run as strided subtrees in one to three launches, the
-// first with 2^split times the default number of CTAs (merkle.cu).  DFT (two-pass sizes): the first pass transforms columns
-// of 2^L1 rows, L1 = (log_h + 1) / 2 + l1_bias.
+// Tree: levels that make >= 2^wide_log nodes run over the whole GPU, one launch
+// each; the remaining S levels run as strided subtrees in one to three launches,
+// the first with 2^split times the default number of CTAs where a CTA can hold
+// its nodes (tree_plan.h).  DFT (two-pass sizes): the first pass transforms
+// columns of 2^L1 rows, L1 = (log_h + 1) / 2 + l1_bias.
 struct TreeTune {
   int wide_log = 15;
   int split = 0;

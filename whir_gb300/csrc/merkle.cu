@@ -12,6 +12,7 @@
 #include "p2_device.cuh"
 #include "p2_lanes.cuh"
 #include "poseidon2_host.h"
+#include "tree_plan.h"
 
 namespace whir {
 namespace gpu {
@@ -495,9 +496,9 @@ __global__ void __launch_bounds__(1024) tree_subtrees(uint32_t *__restrict__ nod
   }
 }
 
-// Default: levels whose step makes at least 2^15 nodes run one thread per
-// node over the whole GPU; the rest (at most 2^16 nodes at the first narrow
-// level) go through tree_subtrees.  Per-size overrides in tree_tune().
+// Default: levels whose step makes at least 2^15 nodes run over the whole GPU
+// (launch_level); the rest (at most 2^16 nodes at the first narrow level) go
+// through tree_subtrees.  Per-size overrides in tree_tune().
 static std::atomic<int> g_tree_tune[41];  // 0: default, else (wide_log << 4) | (split + 2)
 
 TreeTune tree_tune(int log_h) {
@@ -510,14 +511,7 @@ TreeTune tree_tune(int log_h) {
   }
   return t;
 }
-bool tree_tune_valid(int log_h, TreeTune t) {
-  if (t.wide_log < 10 || t.wide_log > 18 || t.split < -1 || t.split > 1) return false;
-  // the narrow part has S <= wide_log levels; both subtree launches hold at
-  // most 512 nodes per CTA (1024 threads)
-  int S = std::min(log_h, t.wide_log);
-  int log_g = std::max(0, std::min(S, (S + t.split) / 2));
-  return S - log_g <= 9 && log_g <= 9;
-}
+bool tree_tune_valid(int log_h, TreeTune t) { return tree_tune_ok(log_h, t.wide_log, t.split); }
 void set_tree_tune(int log_h, TreeTune t) {
   if (log_h < 0 || log_h > 40 || !tree_tune_valid(log_h, t)) return;
   g_tree_tune[log_h].store((t.wide_log << 4) | (t.split + 2), std::memory_order_relaxed);
@@ -545,17 +539,6 @@ static cudaError_t launch_subtrees(uint32_t *nodes, int log_h, int l0, int steps
   return cudaGetLastError();
 }
 
-// log2 of the first launch's subtrees for a narrow part of S levels.  Up to 9
-// levels in two launches; from 10 on three, the first with up to 128 CTAs
-// (one per SM), so that all levels but the first few have at most 8 nodes per
-// CTA (a launch costs 2.5 us, a level 1.9 to 2.4 us on warps and 4.2 on
-// quads; 11 levels: 31.6 us in three launches, 34.7 in two).  A CTA starts
-// with at most 512 nodes.
-static int first_split(int S, int split) {
-  const int g = (S <= 5 ? 0 : S <= 9 ? S / 2 : std::min(7, S - 4)) + split;
-  return std::min(std::max({g, S - 9, 0}), std::min(S, 9));
-}
-
 cudaError_t build_tree(uint32_t *nodes, int log_h, cudaStream_t st, const WaitReport &report,
                        uint32_t *host_root, unsigned int *flag, unsigned int seq) {
   TreeTune tune = tree_tune(log_h);
@@ -567,7 +550,7 @@ cudaError_t build_tree(uint32_t *nodes, int log_h, cudaStream_t st, const WaitRe
                  half, st, report);
   }
   // the remaining S = log_h - l steps (S <= wide_log) in up to three launches
-  const int S = log_h - l, g = first_split(S, tune.split);
+  const int S = log_h - l, g = tree_first_split(S, tune.split);
   const int g2 = g >= 6 ? g - 4 : 0;  // 16 nodes per CTA, if the top has 64 or more
   cudaError_t e;
   if (g == 0) return launch_subtrees(nodes, log_h, l, S, 1, 1, st, host_root, flag, seq);

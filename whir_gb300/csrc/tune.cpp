@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "kernels.h"
+#include "tree_plan.h"
 
 namespace whir {
 
@@ -59,6 +60,8 @@ std::string autotune(Context &ctx, int lo, int hi) {
           t.split = sp;
           if (!gpu::tree_tune_valid(h, t)) continue;
           if (h <= wl && wl != base.wide_log) continue;  // wide_log >= h: the same split
+          const int S = std::min(h, wl);  // a split that cannot move is the default again
+          if (sp != 0 && gpu::tree_first_split(S, sp) == gpu::tree_first_split(S, 0)) continue;
           gpu::set_tree_tune(h, t);
           double ms = time_ms(ctx, a, b, [&] {
             cuda_check(gpu::build_tree(nodes.as<uint32_t>(), h, st, ctx.wait_report()),
