@@ -49,21 +49,18 @@ cudaError_t init_poseidon2_tables() {
   return e;
 }
 
-// Where the tensor-core kernels (merkle_tensor.cu) take over.  Their tiles
-// are 128 rows and 608 of them (760 of nodes) fill the GPU; a tile takes 9.2 us
-// per width-24 permutation alone on its SM and 16.5 us among four, so launches
-// of few tiles per SM gain nothing over one thread per row.  Measured, tensor
-// against thread, us: 16-word rows 2^15 16.9/13.8, 2^16 22.3/24.4, 2^17
-// 36.0/39.7, 2^18 66.0/74.9, 2^19 117/141; 64-word rows 2^15 52.1/50.1, 2^16
-// 70.3/93.9, 2^17 124/156, 2^19 446/577; nodes 2^16 15.9/16.3, 2^17 26.9/26.0,
-// 2^18 44.0/48.8, 2^19 82.9/91.0.  A tensor launch takes an SM's whole register
-// file and thread-per-row launches of these sizes do not, so where several
-// streams share the GPU the lines lie one size above the break-even alone (32
-// jobs of 2^14..2^20 evaluations on 8 streams: 8.95 ms, 9.1 ms with the lines
-// one size lower).
-static bool leaves_on_tensor(size_t n_rows, int row_len) {
-  return n_rows >= (row_len <= 16 ? (size_t)1 << 17 : (size_t)1 << 16);
-}
+// Where the tensor-core kernels (merkle_tensor.cu) take over: at the break-even
+// of launches alone.  Their tiles are 128 rows and 608 of them (760 of nodes)
+// fill the GPU; a tile takes 9.2 us per width-24 permutation alone on its SM and
+// 16.5 us among four, so launches of few tiles per SM gain nothing over one
+// thread per row.  Measured, tensor against thread, us: 16-word rows 2^15
+// 17.2/14.7, 2^16 22.5/25.7, 2^17 36.4/40.7, 2^18 66.4/76.0; 32-word rows 2^15
+// 29.1/26.9, 2^16 38.8/48.8; 64-word rows 2^15 51.7/51.0, 2^16 70.7/94.6, 2^17
+// 123/158, 2^19 442/578; nodes 2^16 17.1/17.3, 2^17 27.9/27.2, 2^18 45.6/50.0.
+// (32 jobs of 2^14..2^20 evaluations on 8 streams: with either line a factor of
+// two off the same within their spread of 3%.)
+static bool leaves_on_tensor(size_t n_rows) { return n_rows >= (size_t)1 << 16; }
+static bool nodes_on_tensor(size_t nodes) { return nodes >= (size_t)1 << 18; }
 // Lanes per row of small launches (0: one thread).  A thread takes a
 // permutation's latency of 8.5 us per chunk however few the rows are, a quad
 // of lanes 4.2 us, a warp 2.1 us; the instructions grow the other way.  us,
@@ -76,9 +73,10 @@ static int leaf_lanes(size_t n_rows) {
 // Lanes per opened path (0: one thread): 13 to 18 permutations follow one
 // another.  us, warp / quad / thread, paths of 16 words and 14 levels mixed
 // with some of 64 and 12: 128 paths 34/51/111, 1024 40/52/101, 2048 62/52/102,
-// 8192 184/68/102, 11264 -/94/102, 16384 -/118/102.
-static int path_lanes(int n) { return n <= 1024 ? 32 : n <= 10240 ? 4 : 0; }
-static bool nodes_on_tensor(size_t nodes) { return nodes >= ((size_t)1 << 17); }
+// 8192 184/68/102.  Quads take CTAs of 32 paths, and their time steps with the
+// CTAs per SM (paths of a proof of 2^16 evaluations, quad / thread): two 73/114,
+// three, up to 14592 paths, 98/114, four 122/114.
+static int path_lanes(int n) { return n <= 1024 ? 32 : n <= 152 * 3 * 32 ? 4 : 0; }
 
 // One row per thread; a row of ROW = 16·c words is c permutations
 // (PaddingFreeSponge: overwrite the 16 rate lanes, permute).  Base rows are
@@ -352,7 +350,7 @@ cudaError_t verify_paths(const PathDesc *d, const uint32_t *words, const uint32_
 cudaError_t hash_rows(const uint32_t *rows, size_t n_rows, int row_len, uint32_t *digests,
                       cudaStream_t st, const WaitReport &report) {
   if (n_rows == 0) return cudaSuccess;
-  if (leaves_on_tensor(n_rows, row_len) && ((uintptr_t)digests & 15) == 0) {
+  if (leaves_on_tensor(n_rows) && ((uintptr_t)digests & 15) == 0) {
     hash_rows_tensor(rows, n_rows, row_len, digests, st, report);
     count_launches(1);
     return cudaGetLastError();
