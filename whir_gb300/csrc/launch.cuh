@@ -5,11 +5,20 @@
 // stream serialisation: on GB300 a chain of dependent kernels of about 10 us
 // each took 10.8 us per kernel this way against 12.3 us with plain launches
 // (the gap between them shrinks from about 2.3 us to under 1 us).  In
-// exchange every kernel of this library begins with pdl_wait(), which returns
-// once the preceding grid in the stream has completed and its memory writes
-// are visible; nothing of the kernel runs before it, so each kernel sees
-// exactly what it would after a plain launch.  (griddepcontrol.wait returns
-// at once in a kernel that was launched without the attribute.)
+// exchange every kernel of this library calls pdl_wait(), which returns once the
+// preceding grid in the stream has completed and its memory writes are visible,
+// before it touches any buffer that another kernel or a copy writes; so each
+// kernel sees exactly what it would after a plain launch.  Most begin with it.
+// Before it a kernel may only fill its own shared and tensor memory, and read
+// its arguments and the tables that init_device_tables writes once per device
+// (the hash kernels on lanes, the path checks and the tree's subtrees load such
+// tables, the tensor-core ones copy theirs and allocate tensor memory).  That
+// early allocation waits for nothing of the grid before: no kernel here triggers
+// its dependents, so a CTA starts after all CTAs of that grid have left and
+// freed theirs; a CTA of another stream's tensor kernel does not share an SM
+// with it (their registers do not fit) and would free its columns by itself.
+// (griddepcontrol.wait returns at once in a kernel that was launched without
+// the attribute.)
 #pragma once
 #include <cuda_runtime.h>
 

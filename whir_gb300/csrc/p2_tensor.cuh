@@ -17,10 +17,10 @@
 // = row, so a thread reads and writes only its own row and no data crosses
 // threads.  A CTA runs as many tiles as an SM's 512 columns hold, four of 128
 // or (width 16) five of 96, which hide one another's waits: a permutation
-// waits for the matrix unit some 20 times, 350 to 400 cycles each.  (Five
+// waits for the matrix unit 15 times (width 16: 17), 350 to 400 cycles each.  (Five
 // tiles against four, 2^18 nodes 49.5 -> 45.1 us, 2^19 87.6 -> 84.4; width 24
-// needs 112 columns at least.)  The tables (86 KB at width 24) are read once
-// per CTA.
+// needs 112 columns at least.)  The tables (95 KB at width 24, 48 KB at 16) are read
+// once per CTA.
 #pragma once
 #include "kernels.h"
 #include "launch.cuh"
