@@ -43,17 +43,17 @@ WORKLOAD = dict(k=24, folding=4, rate=2, initial_reduction=1, soundness="Johnson
 METRIC = "proofs/sec and p50/p99 latency, batched/served vs plain, 1 GB300, bit-exact"
 UNIT = "proofs/s"
 # Per-launch DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of the
-# leaf-hash launches of a k = 24 proof: 0.975 of the algorithmic bytes (307.0 MB
-# per launch), as ncu counted for 2^20 rows of 64 words (268.6 MB read, 26.0 MB
-# written of 302.0 MB; the capture and its command are in profiles/).
-NCU_TRAFFIC_BYTES = {"leaf_hash": 299.4e6}
+# leaf-hash launches of a k = 24 proof, the mean of a proof's five as ncu counted
+# them (1 465.9 MB of 1 535.1 MB algorithmic; the capture and its command are in
+# profiles/).
+NCU_TRAFFIC_BYTES = {"leaf_hash": 293.2e6}
 NCU_TRAFFIC_K = 24
 # Thread instructions per width-24 permutation of the leaf hash
 # (smsp__inst_executed.sum * 32 / permutations of hash_rows_tensor_kernel on
 # 2^20 rows of 64 words, the same ncu summary in profiles/).  With one warp
 # instruction issued per cycle on each of the 4 sub-partitions of each SM,
 # the issue-bound rate is SMs * 4 * 32 * clock / this.
-LEAF_INSTR_PER_PERM24 = 3940
+LEAF_INSTR_PER_PERM24 = 3907
 GB300_SMS = 152
 
 
@@ -808,6 +808,7 @@ def run_gb300(args):
         "roofline": {"kernel": dom, "bound": "hbm", "achieved": achieved, "peak": hbm_peak,
                      "unit": "GB/s", "frac": achieved / hbm_peak if achieved else None,
                      "peak_source": peak_src, "traffic": traffic,
+                     "traffic_source": "ncu dram bytes per launch, an earlier run (profiles/)",
                      "per_launch_ms": per_launch_ms,
                      "limiter": "integer pipes, not HBM: see integer_pipe (frac of the issue "
                                 "bound); this HBM frac only shows the memory side is idle"},

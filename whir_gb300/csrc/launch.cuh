@@ -24,6 +24,8 @@
 
 #include <utility>
 
+#include "gpu_shape.h"
+
 namespace whir {
 namespace gpu {
 

@@ -76,7 +76,7 @@ static int leaf_lanes(size_t n_rows) {
 // 8192 184/68/102.  Quads take CTAs of 32 paths, and their time steps with the
 // CTAs per SM (paths of a proof of 2^16 evaluations, quad / thread): two 73/114,
 // three, up to 14592 paths, 98/114, four 122/114.
-static int path_lanes(int n) { return n <= 1024 ? 32 : n <= 152 * 3 * 32 ? 4 : 0; }
+static int path_lanes(int n) { return n <= 1024 ? 32 : n <= SMS * 3 * 32 ? 4 : 0; }
 
 // One row per thread; a row of ROW = 16·c words is c permutations
 // (PaddingFreeSponge: overwrite the 16 rate lanes, permute).  Base rows are
@@ -639,7 +639,7 @@ cudaError_t interleave_rows(const uint32_t *src, size_t rows, size_t w, int batc
   const bool vec = w % 4 == 0 && (((uintptr_t)src | (uintptr_t)dst) & 15) == 0;
   const size_t items = vec ? total / 4 : total;
   const size_t g = (items + T - 1) / T;
-  const unsigned grid = (unsigned)(g < 152 * 32 ? g : 152 * 32);
+  const unsigned grid = (unsigned)(g < SMS * 32 ? g : SMS * 32);
   if (vec)
     launch(interleave_kernel<uint4>, grid, T, 0, st, reinterpret_cast<const uint4 *>(src), rows,
            w / 4, (size_t)batch, reinterpret_cast<uint4 *>(dst));

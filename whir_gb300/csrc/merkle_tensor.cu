@@ -9,7 +9,6 @@ namespace whir {
 namespace gpu {
 
 namespace {
-constexpr int SMS = 152;
 __device__ uint4 g_tab16[P2Mat<16>::bytes / 16];
 __device__ uint4 g_tab24[P2Mat<24>::bytes / 16];
 
@@ -170,7 +169,7 @@ Tri tri_of(int width) {
 }
 unsigned grid_of(size_t n) {
   const size_t tiles = (n + 127) / 128;
-  return (unsigned)(tiles < SMS ? tiles : SMS);
+  return (unsigned)(tiles < (size_t)SMS ? tiles : SMS);
 }
 }  // namespace
 

@@ -685,7 +685,7 @@ static cudaError_t launch_tile_v(const uint32_t *in, uint32_t *out, int S, size_
         dft_tile_v2<C, 4, 0>, dft_tile_v2<C, 4, 1>, dft_tile_v2<C, 4, 2>, dft_tile_v2<C, 4, 3>};
     static const decltype(&dft_tile_v2<C, 4, 0>) three[4] = {
         dft_tile_v2<C, 3, 0>, dft_tile_v2<C, 3, 1>, dft_tile_v2<C, 3, 2>, dft_tile_v2<C, 3, 3>};
-    const bool full = rows * C * 4 <= (48u << 10) && (size_t)grid.x * grid.y > 3 * 152;
+    const bool full = rows * C * 4 <= (48u << 10) && (size_t)grid.x * grid.y > 3 * SMS;
     launch((full ? four : three)[S < 6 ? 3 : S % 3], grid, threads, rows * C * 4, st, in, out, S, lg, (uint32_t)width,
            (uint32_t)rows_valid, (uint32_t)a_in, (uint32_t)b_in, (uint32_t)a_out,
            (uint32_t)b_out, pre_log, tw_log, ix);
@@ -728,7 +728,7 @@ static cudaError_t tile_any(const uint32_t *in, uint32_t *out, int S, size_t wid
   // 6.9 / 6.4, 2^14 from 2^8 7.0 / 6.6; above, 2^14 of 64 from 2^8 7.4 / 8.6).
   int lg = 0;
   while (S + lg < 10 && ((size_t)2 << lg) <= n_outer) lg++;
-  const bool few = (width / 8) * (n_outer >> lg) <= 76;
+  const bool few = (width / 8) * (n_outer >> lg) <= SMS / 2;
   if (aligned && width % 8 == 0 && !few)
     return launch_tile_v<8>(in, out, S, width, rows_valid, n_outer, a_in, b_in, a_out, b_out,
                             pre_log, tw_log, st);

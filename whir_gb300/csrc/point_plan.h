@@ -3,6 +3,8 @@
 #pragma once
 #include <stddef.h>
 
+#include "gpu_shape.h"
+
 namespace whir {
 namespace gpu {
 
@@ -45,12 +47,12 @@ constexpr size_t POINT_FACTORS = 64 * 16;
 // blocks are 4096 words); the low table and 2^ks columns' sums
 inline PointLaunch compress_hi_point_launch(int k, int ks) {
   const int s_lo = compress_hi_point_low(k, ks);
-  return point_launch((size_t)1 << (k - ks - s_lo), 152 * (ks + s_lo == 12 ? 3 : 4),
+  return point_launch((size_t)1 << (k - ks - s_lo), (size_t)SMS * (ks + s_lo == 12 ? 3 : 4),
                       ((size_t)16 << s_lo) + ((size_t)32 << ks) + POINT_FACTORS);
 }
 // eval_ext_point: blocks of 2^8 entries, eight CTAs per SM
 inline PointLaunch eval_ext_point_launch(int k) {
-  return point_launch((size_t)1 << (k < 8 ? 0 : k - 8), 152 * 8, POINT_FACTORS);
+  return point_launch((size_t)1 << (k < 8 ? 0 : k - 8), (size_t)SMS * 8, POINT_FACTORS);
 }
 
 }  // namespace gpu

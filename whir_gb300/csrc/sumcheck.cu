@@ -440,7 +440,7 @@ cudaError_t compress_hi_batch(const uint32_t *poly, int k, int ks, const E4 *eq_
   size_t n_hi = (size_t)1 << (k - ks - s_lo);
   // about four (three) CTAs per SM over all instances
   const bool pipe = ((size_t)1 << (ks + s_lo)) == 16 * (size_t)CH_T;
-  const size_t per = ((size_t)152 * (pipe ? 3 : 4) + batch - 1) / batch;
+  const size_t per = ((size_t)SMS * (pipe ? 3 : 4) + batch - 1) / batch;
   dim3 grid((unsigned)(n_hi < per ? n_hi : per), (unsigned)batch);
   size_t smem = ((size_t)1 << s_lo) * sizeof(E4) + ((size_t)4 << ks) * 8;
   launch(pipe ? compress_hi_pipe_kernel<false> : compress_hi_kernel<false>, grid, CH_T, smem, st,
@@ -507,7 +507,7 @@ static cudaError_t compress_lo_launch(const uint32_t *poly, int k, int ks, const
   if (ks > 8 || ks > k || batch < 1 || batch > 65535) return cudaErrorInvalidValue;
   size_t n_out = (size_t)1 << (k - ks);
   unsigned T = 256;
-  size_t g = (n_out + T - 1) / T, cap = ((size_t)152 * 16 + batch - 1) / batch;
+  size_t g = (n_out + T - 1) / T, cap = ((size_t)SMS * 16 + batch - 1) / batch;
   dim3 grid((unsigned)(g < cap ? g : cap), (unsigned)batch);
   const bool vec = ks >= 2 && aligned16(poly) && aligned16(out) &&
                    (batch == 1 || poly_stride % 4 == 0);
@@ -558,7 +558,7 @@ cudaError_t add_eq_batch(E4 *w, int k, const E4 *tables, int n_tables, int batch
   int s = k / 2;
   size_t n = (size_t)1 << k;
   unsigned T = 256;
-  size_t g = (n + T - 1) / T, cap = ((size_t)152 * 16 + batch - 1) / batch;
+  size_t g = (n + T - 1) / T, cap = ((size_t)SMS * 16 + batch - 1) / batch;
   dim3 grid((unsigned)(g < cap ? g : cap), (unsigned)batch);
   if (aligned16(w) && aligned16(tables))
     launch(add_eq_kernel<true>, grid, T, 0, st, w, n, s, (size_t)1 << s, (size_t)1 << (k - s),
@@ -1069,7 +1069,7 @@ __global__ void __launch_bounds__(256) round_kernel(const E4 *__restrict__ p_in,
 
 // CTAs of a round over n elements (after the fold): about four per SM at most
 static unsigned round_ctas(size_t n, int batch) {
-  const size_t g = ((n + 1) / 2 + 255) / 256, cap = ((size_t)152 * 4 + batch - 1) / batch;
+  const size_t g = ((n + 1) / 2 + 255) / 256, cap = ((size_t)SMS * 4 + batch - 1) / batch;
   return (unsigned)(g < cap ? (g ? g : 1) : cap);
 }
 static cudaError_t round_launch(const E4 *p_in, const E4 *w_in, size_t n_in, bool fold, E4 r,
@@ -1136,7 +1136,7 @@ cudaError_t eval_ext_batch(const E4 *poly, int k, const E4 *eq_lo, int s_lo, con
                            size_t tab_stride, int batch, unsigned long long *acc,
                            cudaStream_t st, const Publish &pub) {
   if (batch < 1 || batch > 65535 || s_lo > k) return cudaErrorInvalidValue;
-  size_t n_hi = (size_t)1 << (k - s_lo), cap = ((size_t)152 * 8 + batch - 1) / batch;
+  size_t n_hi = (size_t)1 << (k - s_lo), cap = ((size_t)SMS * 8 + batch - 1) / batch;
   dim3 grid((unsigned)(n_hi < cap ? n_hi : cap), (unsigned)batch);
   if (aligned16(poly) && aligned16(eq_lo) && aligned16(eq_hi))
     launch(eval_ext_kernel<true>, grid, 256, 0, st, poly, k, eq_lo, s_lo, eq_hi, acc, pub,
@@ -1211,7 +1211,7 @@ __global__ void __launch_bounds__(256) dot_ext_kernel(const E4 *__restrict__ a,
 cudaError_t dot_ext(const E4 *a, const E4 *b, size_t n, unsigned long long *acc, cudaStream_t st,
                     const Publish &pub) {
   size_t g = (n + 255) / 256;
-  unsigned grid = (unsigned)(g < 152 * 4 ? (g ? g : 1) : 152 * 4);
+  unsigned grid = (unsigned)(g < SMS * 4 ? (g ? g : 1) : SMS * 4);
   if (aligned16(a) && aligned16(b))
     launch(dot_ext_kernel<true>, grid, 256, 0, st, a, b, n, acc, pub);
   else
