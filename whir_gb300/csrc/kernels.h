@@ -101,8 +101,8 @@ cudaError_t gather_openings_val(const uint32_t *rows, int row_len, const uint32_
 // path i's words start at words[d[i].off]: the row (row_len words, hashed as
 // a leaf), then log_h sibling digests bottom-up, as an opening lies in a
 // proof; its root is roots[8 i .. 8 i + 8).  ok[i] = 1 when the path climbs
-// to its root, else 0.  One thread per path; paths sorted by (row_len,
-// log_h) keep warps uniform.  log_h <= 40.
+// to its root, else 0.  A warp, a quad of lanes or a thread per path, by their
+// number; paths sorted by (row_len, log_h) keep warps uniform.  log_h <= 40.
 struct PathDesc {
   uint64_t off;
   uint64_t index;
